@@ -1125,10 +1125,14 @@ static int build_plan(const mi_map_desc &m, const mi_plan_opts &o, Plan *p, Host
         int lo = 0, hi = m.ny;
         while (lo < m.ny && !row[lo]) ++lo;
         while (hi > lo && !row[hi - 1]) --hi;
-        lo &= ~7;
-        // the panel's own width bounds the span: the transpose reads the panel's frame rows
-        if (hi > lo) hi = std::min(p->panels[pi].ny, (hi + 7) & ~7);
-        else hi = lo;
+        // the panel's own width bounds the span: the transpose reads the panel's frame rows.  A
+        // row without references has no span, whatever the width it was looked for in
+        if (hi > lo) {
+          lo &= ~7;
+          hi = std::min(p->panels[pi].ny, (hi + 7) & ~7);
+        } else {
+          lo = hi = 0;
+        }
         span_lo[z] = lo;
         row_off[z] = (int32_t)n_xc;
         for (int y = lo; y < hi; y += kXcChunk)

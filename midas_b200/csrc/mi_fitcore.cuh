@@ -11,6 +11,26 @@ __device__ inline double warp_sum(double v) {
   return v;
 }
 
+// The warp sums of N <= 32 values per lane; lane k returns value k's (lanes >= N: 0).  The
+// butterfly of warp_sum with each step halving the values a lane still carries: 31 shuffles
+// instead of 5 N, and the same additions in the same order, so the same bits.
+template <int N>
+__device__ __forceinline__ double warp_sums(const double *v, int lane) {
+  double t[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) t[k] = k < N ? v[k] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < o; ++k) {
+      const double keep = up ? t[k + o] : t[k], give = up ? t[k] : t[k + o];
+      t[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  return t[0];
+}
+
 // TCH FWHM and mixing from (sig [centi-x^2], gam [centi-x]); also d/dsig, d/dgam
 __device__ inline void tch(float sig, float gam, float *fw, float *eta, float *dfw_ds, float *dfw_dg,
                            float *deta_ds, float *deta_dg) {

@@ -44,8 +44,9 @@ def fit_batch(x: torch.Tensor, lineouts: torch.Tensor, peaks: torch.Tensor, *, m
     F, n_x = lo.shape
     if x.numel() != n_x:
         raise ValueError("x and lineouts disagree in length")
-    out = torch.zeros((F, pk.numel(), L.FIT_NOUT), dtype=torch.float64, device=dev)
-    it = torch.zeros((F, pk.numel()), dtype=torch.int32, device=dev)
+    new = torch.empty if n_x else torch.zeros     # the kernel writes every window of a non-empty axis
+    out = new((F, pk.numel(), L.FIT_NOUT), dtype=torch.float64, device=dev)
+    it = new((F, pk.numel()), dtype=torch.int32, device=dev)
     opts = L.MiFitOpts(MODELS[model], int(half_window), int(max_iter), float(x_bin), float(px_um),
                        float(lsd_um))
     with torch.cuda.device(dev):

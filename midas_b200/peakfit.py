@@ -113,8 +113,8 @@ class FitPlan:
             ld_series = series.stride(0) if series.dim() > 1 else 0
         dt = L.DT_F64 if series.dtype == torch.float64 else L.DT_F32
         tot = n_series * n_sub
-        out = torch.zeros((tot, self.n_peaks, L.FIT_NOUT), dtype=torch.float64, device=series.device)
-        it = torch.zeros((tot, self.n_peaks), dtype=torch.int32, device=series.device)
+        out = torch.empty((tot, self.n_peaks, L.FIT_NOUT), dtype=torch.float64, device=series.device)
+        it = torch.empty((tot, self.n_peaks), dtype=torch.int32, device=series.device)
         with torch.cuda.device(series.device):
             L.check(L.lib().mi_fit_plan_run(self._h, series.data_ptr(), dt, n_series, n_sub, int(ld_series),
                                             int(ld_sub), int(ld_x), out.data_ptr(), it.data_ptr(),

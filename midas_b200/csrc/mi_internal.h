@@ -345,6 +345,22 @@ __host__ __device__ inline MmadBlob mmad_blob_layout(int n_k, int n_terms) {
   return b;
 }
 
+// Bins in slices of 32: blocks of (32 >> ee) R rows x (1 << ee) eta columns, row-major blocks.
+struct PlainLayout {
+  int n_r = 0, n_eta = 0, ee = 0;
+  int64_t n_slices = 0;
+};
+struct PlainFill {
+  const mi_map_record *recs;
+  const int32_t *nmap, *cnt;
+  const int64_t *slice_ptr;
+  uint2 *t2;
+  uint4 *t4;
+  float *area_gs;
+  int ny, nz, mode, sem;
+  float bc_y, bc_z;
+};
+
 struct Plan {
   int device = 0;
   int mode = 0, normalize = 1, semantics = 0;
@@ -403,13 +419,14 @@ struct Plan {
   };
   std::vector<Panel> panels;     // one entry for an ordinary plan
 
-  // plain (reference-layout) path
-  int32_t *d_nmap = nullptr;     // {count, offset} per bin
-  int32_t *d_sorted = nullptr;   // bins, heaviest first
-  int32_t *d_off = nullptr;      // per record: flat pixel offset (floor mode)
-  float *d_w = nullptr, *d_aw = nullptr, *d_dr = nullptr, *d_py = nullptr, *d_pz = nullptr;
+  // plain (one-frame) path: the records slice by slice (mi_plain.cu)
+  PlainLayout plain;
+  int32_t *d_plain_cnt = nullptr;  // records per slice lane
+  int64_t *d_plain_ptr = nullptr;  // first record of each slice
+  uint2 *d_plain_t2 = nullptr;     // floor mode: {pixel or -1, frac}
+  uint4 *d_plain_t4 = nullptr;     // bilinear / gradient: {base pixel, y, z fraction, frac}
+  float *d_area_gs = nullptr;      // per bin: the areaWeights summed in FP32, in record order
   double *d_area_in = nullptr;   // per bin in-bounds area
-  double *d_area_all = nullptr;  // per bin sum of all areaWeight
   float *d_plain_img = nullptr;  // one cast frame
   size_t device_bytes = 0;
 };
@@ -444,6 +461,8 @@ int launch_mmad(Plan *p, const void *frames, int dtype, int F, int64_t stride, f
 int launch_mmad_dark(Plan *p, cudaStream_t s);
 // kernel (c): lineouts of frames [0, n_frames) from the partial sums in `partial`
 int launch_lineout(Plan *p, const double *partial, int n_frames, double *lo_aw, double *lo_sm, cudaStream_t s);
+// device layout of the one-frame path's records (the map's records and {count, offset} pairs)
+int build_plain(Plan *p, const mi_map_record *recs, const int32_t *nmap, size_t *acct);
 int launch_plain(Plan *p, const void *frame, int dtype, double *cake, double *lo_aw,
                  double *lo_sm, cudaStream_t s);
 int launch_cast(const void *frames, int dtype, int64_t n_pixels, int n_frames,

@@ -569,8 +569,8 @@ static int choose_run_len(const HostCSR &csr, const mi_map_desc &m, int rows, in
 static int free_plan_mem(Plan *p) {
   cudaSetDevice(p->device);
   void *ptrs[] = {p->d_blobs, p->d_tiles, p->d_items, p->d_den_aw, p->d_cnt, p->d_partial,
-                  p->d_dark, p->d_err, p->d_nmap, p->d_sorted, p->d_off, p->d_w, p->d_aw,
-                  p->d_dr, p->d_py, p->d_pz, p->d_area_in, p->d_area_all, p->d_plain_img,
+                  p->d_dark, p->d_err, p->d_plain_cnt, p->d_plain_ptr, p->d_plain_t2,
+                  p->d_plain_t4, p->d_area_gs, p->d_area_in, p->d_plain_img,
                   p->d_ctr, p->d_span_lo, p->d_row_off, p->d_xchunks, p->d_xc,
                   p->d_xc_pix, p->d_nan_bins};
   for (void *q : ptrs)
@@ -1315,50 +1315,7 @@ static int build_plan(const mi_map_desc &m, const mi_plan_opts &o, Plan *p, Host
   }
 
   if ((rc = upload(&p->d_area_in, csr.area_in.data(), csr.area_in.size(), &acct))) return rc;
-  // ---- plain path: reference SoA layout (PrecomputeOffsets_kernel, …Stream.cu:901-924)
-  if (!pre) {
-    const int64_t nrec = m.n_records;
-    std::vector<int32_t> off(nrec);
-    std::vector<float> w(nrec), aw(nrec), dr(nrec), py(nrec), pz(nrec);
-#pragma omp parallel for schedule(static)
-    for (int64_t i = 0; i < nrec; ++i) {
-      const mi_map_record &r = m.records[i];
-      long long zz = (long long)r.z;
-      float s = (float)(zz * (long long)m.ny) + r.y;
-      long long o2 = (long long)s;
-      const int64_t ty = (int64_t)r.y, tz = (int64_t)r.z;
-      const bool inb = ty >= 0 && ty < m.ny && tz >= 0 && tz < m.nz;
-      if (p->semantics == MI_SEM_PY) o2 = inb ? (long long)(tz * m.ny + ty) : -1;
-      else if (o2 < 0 || o2 >= (long long)m.ny * m.nz) o2 = -1;
-      off[i] = (int32_t)o2;
-      w[i] = (float)r.frac;
-      aw[i] = r.areaWeight;
-      dr[i] = r.deltaR;
-      py[i] = r.y;
-      pz[i] = r.z;
-    }
-    std::vector<int32_t> sorted(p->n_bins);
-    std::iota(sorted.begin(), sorted.end(), 0);
-    std::stable_sort(sorted.begin(), sorted.end(),
-                     [&](int32_t a, int32_t b) { return m.nmap[2 * a] > m.nmap[2 * b]; });
-    std::vector<double> area_all(p->n_bins, 0.0);
-    for (int64_t b = 0; b < p->n_bins; ++b) {
-      double s = 0;
-      for (int32_t k = 0; k < m.nmap[2 * b]; ++k) s += m.records[(int64_t)m.nmap[2 * b + 1] + k].areaWeight;
-      area_all[b] = s;
-    }
-    if ((rc = upload(&p->d_nmap, m.nmap, (size_t)(2 * p->n_bins), &acct))) return rc;
-    if ((rc = upload(&p->d_sorted, sorted.data(), sorted.size(), &acct))) return rc;
-    if ((rc = upload(&p->d_off, off.data(), off.size(), &acct))) return rc;
-    if ((rc = upload(&p->d_w, w.data(), w.size(), &acct))) return rc;
-    if ((rc = upload(&p->d_aw, aw.data(), aw.size(), &acct))) return rc;
-    if ((rc = upload(&p->d_dr, dr.data(), dr.size(), &acct))) return rc;
-    if ((rc = upload(&p->d_py, py.data(), py.size(), &acct))) return rc;
-    if ((rc = upload(&p->d_pz, pz.data(), pz.size(), &acct))) return rc;
-    if ((rc = upload(&p->d_area_all, area_all.data(), area_all.size(), &acct))) return rc;
-    MI_CUDA(cudaMalloc((void **)&p->d_plain_img, n_pix * sizeof(float)));
-    acct += n_pix * sizeof(float);
-  }
+  if (!pre && (rc = build_plain(p, m.records, m.nmap, &acct))) return rc;
   p->device_bytes = acct;
   return MI_OK;
 }

@@ -218,6 +218,7 @@ constexpr int kXcGroupsF = 2;      // fp32 groups held per launch
 constexpr int kXcRowBytes = 256;   // bytes per compact pixel
 constexpr int kXcChunk = 256;
 constexpr int kUploadRows = 16;   // detector rows per column range of mi_upload_frames
+constexpr int64_t kUploadKernelBytes = 1 << 20;   // per group: up to this, one kernel uploads all groups
 struct XcChunk {
   int32_t z, y0, n, c0;  // detector row, first column, pixels, compact index of the first
 };
@@ -379,6 +380,8 @@ struct Plan {
   // rows, the columns any of its rows references, rounded out to 8 pixels as the transpose
   // reads them: {first row, end row, first column, end column}
   std::vector<int4> upload_groups;
+  int4 *d_upload = nullptr;      // the same on the device
+  int64_t upload_pixels = 0;     // pixels of a frame they hold
 
   // batched path
   uint8_t *d_blobs = nullptr;
@@ -447,6 +450,9 @@ bool runs_uses_xc(const Plan *p, int dtype);
 // `as_f32` is false (8/16-bit frames, F <= 128), else fp32 rows minus the dark (F <= 64).
 int launch_xc(Plan *p, int panel, const void *frames, int dtype, int F, int64_t stride, bool as_f32,
               cudaStream_t s);
+// Upload of page-locked host frames by one kernel; false when it does not apply
+bool launch_upload(const Plan *p, const void *host, int es, int n_frames, int64_t host_stride, void *dev,
+                   int64_t dev_stride, cudaStream_t s);
 // Caking of frames [0, F) (F <= 128 u16 / 64 fp32) already staged pixel-major.
 int launch_runs_staged(Plan *p, bool as_f32, int F, float *cake, double *partial, bool want_lo, cudaStream_t s);
 // MMA encoding (mi_mma.cu): caking of frames [0, F) (F <= 128) staged as byte planes, and

@@ -572,7 +572,7 @@ static int free_plan_mem(Plan *p) {
                   p->d_dark, p->d_err, p->d_plain_cnt, p->d_plain_ptr, p->d_plain_t2,
                   p->d_plain_t4, p->d_area_gs, p->d_area_in, p->d_plain_img,
                   p->d_ctr, p->d_span_lo, p->d_row_off, p->d_xchunks, p->d_xc,
-                  p->d_xc_pix, p->d_nan_bins};
+                  p->d_xc_pix, p->d_nan_bins, p->d_upload};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   return MI_OK;
@@ -1281,6 +1281,8 @@ static int build_plan(const mi_map_desc &m, const mi_plan_opts &o, Plan *p, Host
   if ((rc = upload(&p->d_tiles, tiles.data(), tiles.size(), &acct))) return rc;
   if ((rc = upload(&p->d_items, items_sorted.data(), items_sorted.size(), &acct))) return rc;
   if ((rc = upload(&p->d_den_aw, den.data(), den.size(), &acct))) return rc;
+  if ((rc = upload(&p->d_upload, p->upload_groups.data(), p->upload_groups.size(), &acct))) return rc;
+  for (const int4 &g : p->upload_groups) p->upload_pixels += (int64_t)(g.y - g.x) * (g.w - g.z);
   if ((rc = upload(&p->d_cnt, cnt.data(), cnt.size(), &acct))) return rc;
 
   {
@@ -1748,8 +1750,7 @@ int mi_plan_get_info(const mi_plan *p, mi_plan_info *info) {
   info->xc_pixels = p->n_xc;
   info->ref_row_lo = p->ref_row_lo;
   info->ref_row_hi = p->ref_row_hi;
-  info->upload_pixels = 0;
-  for (const int4 &g : p->upload_groups) info->upload_pixels += (int64_t)(g.y - g.x) * (g.w - g.z);
+  info->upload_pixels = p->upload_pixels;
   return MI_OK;
 }
 
@@ -1889,6 +1890,8 @@ int mi_upload_frames(const mi_plan *p, const void *host, int dtype, int n_frames
   if (!p->upload_groups.empty() && host_stride % p->ny == 0 && device_stride % p->ny == 0) {
     // one 3-D copy per row group: its referenced columns x its rows x the frames, so only
     // the referenced part of each row crosses PCIe (a frame is host_stride / ny rows deep)
+    if (launch_upload(p, host, (int)es, n_frames, host_stride, device_frames, device_stride, (cudaStream_t)stream))
+      return MI_OK;
     const size_t pitch = (size_t)p->ny * es;
     for (const int4 &g : p->upload_groups) {
       cudaMemcpy3DParms c = {};

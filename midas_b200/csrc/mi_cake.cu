@@ -365,7 +365,10 @@ int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t st
   a.err = p->d_err;
   if (!a.want_cake && !a.want_lo) return MI_OK;
   int rc = MI_OK;
-  if (p->encoding == MI_ENC_MMA) {
+  if (p->d_one_terms && n_frames <= kOneFrames) {
+    // few frames: a lane per bin, the same sums (mi_one.cu)
+    rc = launch_one(p, frames, dtype, n_frames, stride, cake, partial, a.want_lo, s);
+  } else if (p->encoding == MI_ENC_MMA) {
     // kernel (a) splits a chunk of frames into byte planes, then kernel (b) on the tensor cores
     if (!(dtype == MI_DT_U16 || dtype == MI_DT_U8))
       return set_error(MI_E_UNSUPPORTED, "MMA plans cake 8/16-bit frames only (dtype %d)", dtype);

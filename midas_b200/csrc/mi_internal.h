@@ -351,6 +351,45 @@ struct PlainLayout {
   int n_r = 0, n_eta = 0, ee = 0;
   int64_t n_slices = 0;
 };
+constexpr int kPlainDeep = 32;   // slices (warps) per SM up to which a lane keeps twice the loads in flight
+inline PlainLayout plain_layout(int n_r, int n_eta) {
+  PlainLayout g;
+  g.n_r = n_r;
+  g.n_eta = n_eta;
+  g.ee = n_eta >= 4 ? 2 : (n_eta >= 2 ? 1 : 0);
+  const int64_t per_row = (n_eta + (1 << g.ee) - 1) >> g.ee;
+  g.n_slices = per_row * ((n_r + (32 >> g.ee) - 1) / (32 >> g.ee));
+  return g;
+}
+#ifdef __CUDACC__
+// the bin of a slice's lane, -1 outside the grid
+__device__ __forceinline__ int64_t plain_bin(const PlainLayout &g, int64_t slice, int lane) {
+  const int64_t per_row = (g.n_eta + (1 << g.ee) - 1) >> g.ee;
+  const int64_t r = (slice / per_row) * (32 >> g.ee) + (lane >> g.ee);
+  const int64_t e = ((slice % per_row) << g.ee) + (lane & ((1 << g.ee) - 1));
+  return r < g.n_r && e < g.n_eta ? r * g.n_eta + e : -1;
+}
+
+// offset (in records) of this lane's record at the current step; moves `at` past the step
+__device__ __forceinline__ int64_t plain_step(bool active, int lane, int64_t &at) {
+  const uint32_t m = __ballot_sync(0xffffffffu, active);
+  const int64_t o = at + __popc(m & ((1u << lane) - 1u));
+  at += __popc(m);
+  return o;
+}
+
+// U records of a lane: loads of inactive lanes go to the slice's first record, so no load waits
+// behind a branch
+template <typename R, int U>
+__device__ __forceinline__ void plain_load(const R *t, int64_t first, int k, int n, int lane, int64_t &at, R *r) {
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const bool active = k + u < n;
+    const int64_t o = plain_step(active, lane, at);
+    r[u] = __ldg(t + (active ? o : first));
+  }
+}
+#endif
 struct PlainFill {
   const mi_map_record *recs;
   const int32_t *nmap, *cnt;
@@ -405,6 +444,14 @@ struct Plan {
   int n_sms = 0;
   int mma_stages = 8, mma_producers = 6;   // pipeline of the MMA kernel (mi_plan_set_mma_pipeline)
 
+  // few frames of the run and CSR encodings (mi_one.cu): terms slice by slice
+  PlainLayout one;
+  int32_t *d_one_cnt = nullptr;
+  int64_t *d_one_ptr = nullptr;
+  uint2 *d_one_terms = nullptr;    // {pixel | kOneEnd, weight}
+  double *d_one_scale = nullptr;   // per bin
+  double *d_one_res = nullptr;     // bin results of kOneChunk frames, for the lineouts
+
   // pixel-major staging (run encoding with 64-frame groups)
   int64_t n_xc = 0;              // compact pixels (0: not built)
   int32_t *d_span_lo = nullptr;  // per detector row: first column of its span
@@ -442,6 +489,16 @@ int build_host_csr(const mi_map_desc &m, int mode, int semantics, HostCSR *out);
 // or a caller-provided array of that size)
 int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t stride,
                 float *cake, double *lo_aw, double *lo_sm, double *partial, cudaStream_t s);
+// Up to kOneFrames frames of a run or CSR plan with a lane per bin (mi_one.cu); the same bits.
+// Run kernel / this, us: 16 frames 311 / 110 (1024^2, 495 x 45), 975 / 369 (2048^2, 990 x 72), 1101 /
+// 640 (2048^2, 1980 x 180 gradient), 1621 / 1114 (2880^2, 3960 x 360 gradient); 32 frames 318 / 218,
+// 996 / 765, 1131 / 1241, 1675 / 2201.  CSR kernel / this, 16 frames: 139 / 91, 703 / 291, 1036 / 413,
+// 1807 / 784.
+constexpr int kOneFrames = 16;
+constexpr int kOneChunk = 8;     // frames whose bin results are held for the lineouts
+int build_one(Plan *p, size_t *acct);
+int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
+               bool want_lo, cudaStream_t s);
 int launch_runs(Plan *p, const void *frames, int dtype, int n_frames, int64_t stride, float *cake, double *partial,
                 bool want_lo, cudaStream_t s);
 // true when launch_runs stages this dtype through the pixel-major buffer

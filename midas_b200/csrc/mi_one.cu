@@ -1,0 +1,416 @@
+// mi_one.cu -- kernel (b) for a few frames: the run and CSR encodings' sums, thread per bin.
+//
+// The batched kernels' lanes are frames: one frame leaves 31 of 32 lanes idle, and their cost is
+// per pass over the map.  Here a lane is a bin.  A bin's terms {pixel, weight} are the ones of
+// the plan's tiles in the order in which the batched kernel adds them, with the ends of its
+// unit partials marked, so every FP64 sum, every rounding of a partial to FP32 and the scaling
+// are the batched kernel's: a frame's cake and lineouts are the same bits on either path.  (A
+// pixel that is not finite reaches the bins whose terms hold it; the run kernel's zero weights
+// spread it to other bins of the same strip.)
+//
+// Layout: slices of 32 neighbouring bins as in the plain path (PlainLayout): step k holds term k
+// of each bin that has one, side by side, nothing padded, 8 B a term.  It is made on the device
+// from the tile blobs when the plan is.
+#include <stdint.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "mi_internal.h"
+
+namespace mi {
+
+constexpr uint32_t kOneEnd = 0x80000000u;   // the term ends a unit partial
+
+// The terms of one bin in summing order.  Run encoding: the units of the bin's strip, records in
+// order, the record's weight for the bin's row where it is not zero.
+struct OneTerms {
+  const uint8_t *blob;
+  TileHdr h;
+  int enc, G, L, i, s;          // row and strip (column) in the tile
+  uint32_t o_rsp, o_up, o_lc, o_w;
+  int u, u_end, j, j1, q;       // unit, its end; record, end of its range; rs of the record
+  __device__ void open(const uint8_t *b, int enc_, int G_, int L_, int row, int col) {
+    blob = b;
+    enc = enc_;
+    G = G_;
+    L = L_;
+    h = *(const TileHdr *)blob;
+    i = row;
+    s = col;
+    uint32_t t0, t1, t2;
+    if (enc == MI_ENC_RUNS) {
+      runs_blob_layout(h.nb, h.n_cols, h.nnz, h.n_u, G, L, &o_rsp, &t0, &t1, &o_up, &o_lc, &o_w);
+      const uint32_t st = ((const uint32_t *)(blob + kRunUnitsOff + kRunWarps * 8))[s];
+      u = (int)(st & 0xFFFF) - 1;
+      u_end = u + 1 + (int)(st >> 16);
+      j = j1 = 0;
+    } else {
+      uint32_t o_rp;
+      blob_layout(h.nb, h.nnz, h.n_u, &o_rp, &t0, &t1, &o_up, &o_lc, &o_w, &t2);
+      const uint32_t *rp = (const uint32_t *)(blob + o_rp) + i * h.n_cols + s;
+      j = (int)rp[0];
+      j1 = (int)rp[1];
+    }
+  }
+  // the next term; false when there is none.  new_unit: the term is the first of its unit
+  __device__ bool next(uint32_t *pix, float *w, bool *new_unit) {
+    const uint16_t *lcol = (const uint16_t *)(blob + o_lc);
+    const uint32_t *upix = (const uint32_t *)(blob + o_up);
+    *new_unit = false;
+    if (enc != MI_ENC_RUNS) {
+      if (j >= j1) return false;
+      *pix = upix[lcol[j]];
+      *w = ((const float *)(blob + o_w))[j];
+      ++j;
+      return true;
+    }
+    const int NRS = G - L + 2;
+    const uint16_t *rp = (const uint16_t *)(blob + o_rsp) + s * NRS;
+    const int q0 = max(0, i - L + 1), q1 = min(i, G - L);   // records whose rows cover row i
+    for (;;) {
+      while (j >= j1) {
+        if (++u >= u_end) return false;
+        const uint16_t *ud = (const uint16_t *)(blob + kRunUnitsOff) + 4 * u;
+        j = max((int)ud[1], (int)rp[q0]);
+        j1 = min((int)ud[2], (int)rp[q1 + 1]);
+        q = q0;
+        *new_unit = true;
+      }
+      while (j >= (int)rp[q + 1]) ++q;
+      const float v = ((const float *)(blob + o_w))[(int64_t)j * L + (i - q)];
+      const int jj = j++;
+      if (v != 0.0f) {
+        *pix = upix[lcol[jj]];
+        *w = v;
+        return true;
+      }
+    }
+  }
+};
+
+struct OneBuild {
+  PlainLayout g;
+  const TileRef *tiles;
+  const uint8_t *blobs;
+  int32_t *tile_of_bin;
+  int32_t *cnt;
+  int64_t *slice_n;
+  const int64_t *slice_ptr;
+  uint2 *terms;
+  double *scale;
+  int n_tiles, enc, G, L;
+};
+
+__global__ void k_one_tiles(OneBuild a) {
+  const int t = blockIdx.x;
+  const TileHdr h = *(const TileHdr *)(a.blobs + a.tiles[t].off);
+  for (int b = threadIdx.x; b < h.nb; b += blockDim.x)
+    a.tile_of_bin[(int64_t)(h.r0 + b / h.n_cols) * a.g.n_eta + h.e0 + b % h.n_cols] = t;
+}
+
+__device__ inline bool one_open(const OneBuild &a, int64_t b, OneTerms *it) {
+  if (b < 0) return false;
+  const uint8_t *blob = a.blobs + a.tiles[a.tile_of_bin[b]].off;
+  const TileHdr h = *(const TileHdr *)blob;
+  it->open(blob, a.enc, a.G, a.L, (int)(b / a.g.n_eta) - h.r0, (int)(b % a.g.n_eta) - h.e0);
+  return true;
+}
+
+__global__ void k_one_count(OneBuild a) {
+  const int lane = threadIdx.x & 31;
+  const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (s >= a.g.n_slices) return;
+  const int64_t b = plain_bin(a.g, s, lane);
+  OneTerms it;
+  int n = 0;
+  if (one_open(a, b, &it)) {
+    uint32_t pix;
+    float w;
+    bool first;
+    while (it.next(&pix, &w, &first)) ++n;
+  }
+  a.cnt[s * 32 + lane] = n;
+  int64_t t = n;
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) a.slice_n[s] = t;
+}
+
+__global__ void k_one_fill(OneBuild a) {
+  const int lane = threadIdx.x & 31;
+  const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (s >= a.g.n_slices) return;
+  const int64_t b = plain_bin(a.g, s, lane);
+  const int n = a.cnt[s * 32 + lane];
+  int64_t at = a.slice_ptr[s];
+  OneTerms it;
+  uint32_t pix = 0;
+  float w = 0.0f;
+  bool first = false, more = one_open(a, b, &it);
+  if (more) {
+    uint32_t o0, o1, o2, o3, o4, o5, o6;
+    if (a.enc == MI_ENC_RUNS) runs_blob_layout(it.h.nb, it.h.n_cols, it.h.nnz, it.h.n_u, a.G, a.L, &o0, &o1, &o2, &o3, &o4, &o5);
+    else blob_layout(it.h.nb, it.h.nnz, it.h.n_u, &o0, &o1, &o2, &o3, &o4, &o5, &o6);
+    a.scale[b] = ((const double *)(it.blob + o1))[it.i * it.h.n_cols + it.s];
+    more = it.next(&pix, &w, &first);
+  }
+  for (int k = 0; __any_sync(0xffffffffu, k < n); ++k) {
+    const int64_t o = plain_step(k < n, lane, at);
+    if (k >= n) continue;
+    uint2 t = make_uint2(pix, __float_as_uint(w));
+    more = it.next(&pix, &w, &first);
+    if (a.enc == MI_ENC_RUNS && (!more || first)) t.x |= kOneEnd;
+    a.terms[o] = t;
+  }
+}
+
+struct OneArgs {
+  PlainLayout g;
+  const uint2 *terms;
+  const int32_t *cnt;
+  const int64_t *slice_ptr;
+  const double *scale;
+  const void *frames;
+  int64_t stride;
+  const float *dark;        // null: none
+  float *cake;              // [F][n_bins] or null
+  double *res;              // [F][n_bins] for the lineouts, or null
+  int64_t n_bins;
+  int F, round_res;         // round_res: the lineouts take the rounded bin results (CSR encoding)
+};
+
+// NF frames per pass over the map, U terms in flight per lane and as many fetched ahead.  Bounded
+// by the gathers (about one lane a clock and SM where a warp's pixels lie in different lines) and
+// at few bins by their latency.  One frame, cake only, where the run kernel took 298, 936, 1038 and
+// 1525 us: 33, 48, 67 and 112 us (1024^2, 495 x 45; 2048^2, 990 x 72; 1980 x 180 gradient; 2880^2,
+// 3960 x 360 gradient, 308 MB of terms).
+template <typename T, int NF, int U>
+__global__ void __launch_bounds__(128) k_one(OneArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= a.g.n_slices) return;
+  const int64_t s = a.g.n_slices - 1 - i;   // outer rings hold more terms: they start first
+  const int64_t b = plain_bin(a.g, s, lane);
+  const int n = a.cnt[s * 32 + lane];
+  int n_max = n;
+  for (int o = 16; o > 0; o >>= 1) n_max = max(n_max, __shfl_xor_sync(0xffffffffu, n_max, o));
+  const int64_t first = a.slice_ptr[s];
+  int64_t at = first;
+  const int f0 = (int)blockIdx.y * NF;
+  const T *img[NF];
+  double acc[NF], tot[NF];
+#pragma unroll
+  for (int q = 0; q < NF; ++q) {
+    img[q] = (const T *)a.frames + (int64_t)min(f0 + q, a.F - 1) * a.stride;
+    acc[q] = tot[q] = 0.0;
+  }
+  uint2 t[U];
+  if (n_max > 0) plain_load<uint2, U>(a.terms, first, 0, n, lane, at, t);
+  for (int k = 0; k < n_max; k += U) {
+    uint2 tn[U];
+    if (k + U < n_max) plain_load<uint2, U>(a.terms, first, k + U, n, lane, at, tn);
+    T raw[U][NF];
+    float d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t p = t[u].x & ~kOneEnd;
+#pragma unroll
+      for (int q = 0; q < NF; ++q) raw[u][q] = __ldg(img[q] + p);
+      d[u] = a.dark ? __ldg(a.dark + p) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const double w = (double)__uint_as_float(t[u].y);
+      const bool in = k + u < n;
+#pragma unroll
+      for (int q = 0; q < NF; ++q) {
+        const double x = fma(w, (double)((float)raw[u][q] - d[u]), acc[q]);
+        acc[q] = in ? x : acc[q];
+      }
+      if (in && (t[u].x & kOneEnd)) {
+#pragma unroll
+        for (int q = 0; q < NF; ++q) {
+          tot[q] += (double)(float)acc[q];
+          acc[q] = 0.0;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) t[u] = tn[u];
+  }
+  if (b < 0) return;
+  const double sc = a.scale[b];
+#pragma unroll
+  for (int q = 0; q < NF; ++q) {
+    if (f0 + q >= a.F) break;
+    const double o = (tot[q] + acc[q]) * sc;   // one of the two is zero
+    const int64_t at_bin = (int64_t)(f0 + q) * a.n_bins + b;
+    if (a.cake) a.cake[at_bin] = (float)o;
+    if (a.res) a.res[at_bin] = a.round_res ? (double)(float)o : o;
+  }
+}
+
+// Lineout partials of the items' rows from the bin results, in the batched kernels' order: a
+// tile's columns in order, then the tiles.  One thread per (frame, item, row).
+__global__ void k_one_partials(const WorkItem *items, int n_items, const TileRef *tiles, const uint8_t *blobs, int enc,
+                               int G, int L, int rows, const double *res, int64_t n_bins, int n_r, int n_eta,
+                               int n_slots, double *partial) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (int64_t)n_items * rows) return;
+  const int64_t f = blockIdx.y;
+  const WorkItem it = items[t / rows];
+  const int r = it.r0 + (int)(t % rows);
+  if (r >= it.r0 + it.n_rows) return;
+  double paw = 0.0, psm = 0.0;
+  for (int k = it.tile_begin; k < it.tile_end; ++k) {
+    const uint8_t *blob = blobs + tiles[k].off;
+    const TileHdr h = *(const TileHdr *)blob;
+    if (r < h.r0 || r >= h.r0 + h.n_rows) continue;
+    uint32_t o0, o1, o_lw, o3, o4, o5, o6;
+    if (enc == MI_ENC_RUNS) runs_blob_layout(h.nb, h.n_cols, h.nnz, h.n_u, G, L, &o0, &o1, &o_lw, &o3, &o4, &o5);
+    else blob_layout(h.nb, h.nnz, h.n_u, &o0, &o1, &o_lw, &o3, &o4, &o5, &o6);
+    const float *lw = (const float *)(blob + o_lw) + (r - h.r0) * h.n_cols;
+    const double *v = res + f * n_bins + (int64_t)r * n_eta + h.e0;
+    double saw = 0.0, ssm = 0.0;
+    for (int c = 0; c < h.n_cols; ++c) {
+      const double o = v[c];
+      const float l = lw[c];
+      saw += o * (double)l;
+      ssm += (l > 0.0f) ? o : 0.0;
+    }
+    paw += saw;
+    psm += ssm;
+  }
+  double *dst = partial + ((f * n_r + r) * n_slots + it.slot) * 2;
+  dst[0] = paw;
+  dst[1] = psm;
+}
+
+int build_one(Plan *p, size_t *acct) {
+  p->one = plain_layout(p->n_r, p->n_eta);
+  const PlainLayout &g = p->one;
+  if (p->n_tiles == 0 || (p->encoding != MI_ENC_RUNS && p->encoding != MI_ENC_CSR)) return MI_OK;
+  cudaStream_t st = nullptr;
+  MI_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  std::vector<void *> tmp;
+  auto temp = [&](void **q, size_t bytes) {
+    cudaError_t e = cudaMallocAsync(q, std::max<size_t>(bytes, 16), st);
+    if (e == cudaSuccess) tmp.push_back(*q);
+    return e;
+  };
+  auto keep = [&](void **q, size_t bytes) {
+    *acct += std::max<size_t>(bytes, 16);
+    return cudaMalloc(q, std::max<size_t>(bytes, 16));
+  };
+  auto build = [&]() -> int {
+    OneBuild a{};
+    a.g = g;
+    a.tiles = p->d_tiles;
+    a.blobs = p->d_blobs;
+    a.n_tiles = p->n_tiles;
+    a.enc = p->encoding;
+    a.G = p->run_g;
+    a.L = p->run_l;
+    MI_CUDA(temp((void **)&a.tile_of_bin, sizeof(int32_t) * p->n_bins));
+    MI_CUDA(temp((void **)&a.slice_n, sizeof(int64_t) * g.n_slices));
+    MI_CUDA(keep((void **)&p->d_one_cnt, sizeof(int32_t) * 32 * g.n_slices));
+    MI_CUDA(keep((void **)&p->d_one_ptr, sizeof(int64_t) * g.n_slices));
+    MI_CUDA(keep((void **)&p->d_one_scale, sizeof(double) * p->n_bins));
+    MI_CUDA(keep((void **)&p->d_one_res, sizeof(double) * p->n_bins * kOneChunk));
+    a.cnt = p->d_one_cnt;
+    a.scale = p->d_one_scale;
+    const unsigned blocks = (unsigned)((g.n_slices * 32 + 127) / 128);
+    k_one_tiles<<<(unsigned)p->n_tiles, 128, 0, st>>>(a);
+    MI_CUDA(cudaGetLastError());
+    k_one_count<<<blocks, 128, 0, st>>>(a);
+    MI_CUDA(cudaGetLastError());
+    std::vector<int64_t> n(g.n_slices);
+    MI_CUDA(cudaMemcpyAsync(n.data(), a.slice_n, sizeof(int64_t) * g.n_slices, cudaMemcpyDeviceToHost, st));
+    MI_CUDA(cudaStreamSynchronize(st));
+    int64_t total = 0;
+    for (int64_t &v : n) {
+      const int64_t c = v;
+      v = total;
+      total += c;
+    }
+    MI_CUDA(cudaMemcpyAsync(p->d_one_ptr, n.data(), sizeof(int64_t) * g.n_slices, cudaMemcpyHostToDevice, st));
+    MI_CUDA(keep((void **)&p->d_one_terms, sizeof(uint2) * total));
+    a.slice_ptr = p->d_one_ptr;
+    a.terms = p->d_one_terms;
+    k_one_fill<<<blocks, 128, 0, st>>>(a);
+    MI_CUDA(cudaGetLastError());
+    MI_CUDA(cudaStreamSynchronize(st));
+    return MI_OK;
+  };
+  const int rc = build();
+  for (void *q : tmp) cudaFreeAsync(q, st);
+  cudaStreamSynchronize(st);
+  cudaStreamDestroy(st);
+  return rc;
+}
+
+template <typename T>
+static int launch_one_t(Plan *p, const OneArgs &a, cudaStream_t s) {
+  const unsigned bx = (unsigned)((p->one.n_slices * 32 + 127) / 128);
+  const bool deep = p->one.n_slices < kPlainDeep * (int64_t)std::max(p->n_sms, 1);
+  if (a.F == 1) {
+    if (deep) k_one<T, 1, 16><<<dim3(bx, 1), 128, 0, s>>>(a);
+    else k_one<T, 1, 8><<<dim3(bx, 1), 128, 0, s>>>(a);
+  } else if (a.F == 2) {
+    k_one<T, 2, 8><<<dim3(bx, 1), 128, 0, s>>>(a);
+  } else {
+    k_one<T, 4, 4><<<dim3(bx, (unsigned)((a.F + 3) / 4)), 128, 0, s>>>(a);
+  }
+  MI_CUDA(cudaGetLastError());
+  return MI_OK;
+}
+
+static int launch_one_chunk(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
+                            bool want_lo, cudaStream_t s) {
+  OneArgs a;
+  a.g = p->one;
+  a.terms = p->d_one_terms;
+  a.cnt = p->d_one_cnt;
+  a.slice_ptr = p->d_one_ptr;
+  a.scale = p->d_one_scale;
+  a.frames = frames;
+  a.stride = stride;
+  a.dark = p->has_dark ? p->d_dark : nullptr;
+  a.cake = cake;
+  a.res = want_lo ? p->d_one_res : nullptr;
+  a.n_bins = p->n_bins;
+  a.F = F;
+  a.round_res = p->encoding == MI_ENC_CSR;
+  int rc = MI_OK;
+  switch (dtype) {
+    case MI_DT_U8: rc = launch_one_t<uint8_t>(p, a, s); break;
+    case MI_DT_U16: rc = launch_one_t<uint16_t>(p, a, s); break;
+    case MI_DT_U32: rc = launch_one_t<uint32_t>(p, a, s); break;
+    case MI_DT_I64: rc = launch_one_t<int64_t>(p, a, s); break;
+    case MI_DT_F32: rc = launch_one_t<float>(p, a, s); break;
+    case MI_DT_F64: rc = launch_one_t<double>(p, a, s); break;
+    case MI_DT_I32: rc = launch_one_t<int32_t>(p, a, s); break;
+    default: return set_error(MI_E_ARG, "unknown dtype %d", dtype);
+  }
+  if (rc || !want_lo) return rc;
+  const int rows = p->lim.rows;
+  const int64_t n = (int64_t)p->n_items * rows;
+  k_one_partials<<<dim3((unsigned)((n + 127) / 128), (unsigned)F), 128, 0, s>>>(
+      p->d_items, p->n_items, p->d_tiles, p->d_blobs, p->encoding, p->run_g, p->run_l, rows, p->d_one_res, p->n_bins,
+      p->n_r, p->n_eta, p->n_slots, partial);
+  MI_CUDA(cudaGetLastError());
+  return MI_OK;
+}
+
+int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
+               bool want_lo, cudaStream_t s) {
+  const size_t es = dtype_size(dtype);
+  int rc = MI_OK;
+  for (int f0 = 0; f0 < F && rc == MI_OK; f0 += kOneChunk)
+    rc = launch_one_chunk(p, (const uint8_t *)frames + (size_t)f0 * stride * es, dtype, std::min(kOneChunk, F - f0),
+                          stride, cake ? cake + (size_t)f0 * p->n_bins : nullptr,
+                          partial + (size_t)f0 * p->n_r * p->n_slots * 2, want_lo, s);
+  return rc;
+}
+
+}  // namespace mi

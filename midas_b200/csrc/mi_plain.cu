@@ -142,21 +142,6 @@ int launch_cast(const void *frames, int dtype, int64_t n_pixels, int n_frames, c
 // of 4 x 8 bins measured 58 / 77 / 102 us, rows of 32 columns 97 / 81 / 147 (before the records
 // were fetched ahead: 52 / 79 / 90).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int64_t plain_bin(const PlainLayout &g, int64_t slice, int lane) {
-  const int64_t per_row = (g.n_eta + (1 << g.ee) - 1) >> g.ee;
-  const int64_t r = (slice / per_row) * (32 >> g.ee) + (lane >> g.ee);
-  const int64_t e = ((slice % per_row) << g.ee) + (lane & ((1 << g.ee) - 1));
-  return r < g.n_r && e < g.n_eta ? r * g.n_eta + e : -1;
-}
-
-// offset (in records) of this lane's record at the current step; moves `at` past the step
-__device__ __forceinline__ int64_t plain_step(bool active, int lane, int64_t &at) {
-  const uint32_t m = __ballot_sync(0xffffffffu, active);
-  const int64_t o = at + __popc(m & ((1u << lane) - 1u));
-  at += __popc(m);
-  return o;
-}
-
 __global__ void k_plain_count(PlainLayout g, const int32_t *nmap, int32_t *cnt, int64_t *slice_n) {
   const int lane = threadIdx.x & 31;
   const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -215,8 +200,6 @@ __global__ void k_plain_fill(PlainLayout g, PlainFill f) {
   if (b >= 0) f.area_gs[b] = A;
 }
 
-constexpr int kPlainDeep = 32;   // slices (warps) per SM
-
 struct PlainArgs {
   PlainLayout g;
   const uint2 *t2;
@@ -229,18 +212,6 @@ struct PlainArgs {
   double *cake;
   int ny, sem, normalize;
 };
-
-// U records of a lane: loads of inactive lanes go to the slice's first record, so no load waits
-// behind a branch
-template <typename R, int U>
-__device__ __forceinline__ void plain_load(const R *t, int64_t first, int k, int n, int lane, int64_t &at, R *r) {
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const bool active = k + u < n;
-    const int64_t o = plain_step(active, lane, at);
-    r[u] = __ldg(t + (active ? o : first));
-  }
-}
 
 // U: records whose pixels a lane has in flight, with as many records fetched ahead
 template <bool FLOOR, int U>
@@ -306,12 +277,8 @@ __global__ void __launch_bounds__(128) k_plain_integrate(PlainArgs a) {
 // The one-frame path's records, laid out on the device from the map's.  On a stream of its own
 // with stream-ordered scratch: a plan made while a server runs must not wait for the device.
 int build_plain(Plan *p, const mi_map_record *recs, const int32_t *nmap, size_t *acct) {
-  PlainLayout &g = p->plain;
-  g.n_r = p->n_r;
-  g.n_eta = p->n_eta;
-  g.ee = p->n_eta >= 4 ? 2 : (p->n_eta >= 2 ? 1 : 0);
-  const int64_t per_row = (p->n_eta + (1 << g.ee) - 1) >> g.ee;
-  g.n_slices = per_row * ((p->n_r + (32 >> g.ee) - 1) / (32 >> g.ee));
+  p->plain = plain_layout(p->n_r, p->n_eta);
+  const PlainLayout &g = p->plain;
   const int64_t n_pix = (int64_t)p->ny * p->nz;
   cudaStream_t st = nullptr;
   MI_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));

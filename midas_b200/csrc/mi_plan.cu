@@ -572,7 +572,8 @@ static int free_plan_mem(Plan *p) {
                   p->d_dark, p->d_err, p->d_plain_cnt, p->d_plain_ptr, p->d_plain_t2,
                   p->d_plain_t4, p->d_area_gs, p->d_area_in, p->d_plain_img,
                   p->d_ctr, p->d_span_lo, p->d_row_off, p->d_xchunks, p->d_xc,
-                  p->d_xc_pix, p->d_nan_bins, p->d_upload};
+                  p->d_xc_pix, p->d_nan_bins, p->d_upload,
+                  p->d_one_cnt, p->d_one_ptr, p->d_one_terms, p->d_one_scale, p->d_one_res};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   return MI_OK;
@@ -1318,6 +1319,7 @@ static int build_plan(const mi_map_desc &m, const mi_plan_opts &o, Plan *p, Host
 
   if ((rc = upload(&p->d_area_in, csr.area_in.data(), csr.area_in.size(), &acct))) return rc;
   if (!pre && (rc = build_plain(p, m.records, m.nmap, &acct))) return rc;
+  if (p->panels.size() == 1 && (rc = build_one(p, &acct))) return rc;
   p->device_bytes = acct;
   return MI_OK;
 }

@@ -1,0 +1,52 @@
+"""A few frames through the lane-per-bin kernel: the same bits as the batched kernel gives those
+frames within a batch of more than 16, for both encodings, frame types, strips of 8, 16 and 32
+rows, variance weights, OpenMP semantics, grids that do not fill a slice, and 1 to 16 frames."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from midas_b200.bin_io import PixelMap, PXLIST_DTYPE
+from midas_b200.kernels import CakePlan
+
+pytestmark = pytest.mark.gpu
+
+
+def _map(n_r, n_eta, ny, nz, seed):
+    rng = np.random.default_rng(seed)
+    counts = rng.integers(0, 25, n_r * n_eta).astype(np.int32)
+    counts[rng.random(counts.size) < 0.1] = 0
+    counts[0] = 90
+    offsets = (np.cumsum(counts) - counts).astype(np.int32)
+    recs = np.zeros(int(counts.sum()), PXLIST_DTYPE)
+    recs["y"], recs["z"] = rng.uniform(-1, ny, recs.size), rng.uniform(-1, nz, recs.size)
+    recs["frac"] = rng.uniform(0.1, 1.0, recs.size)
+    recs["areaWeight"], recs["deltaR"] = recs["frac"], rng.uniform(-0.5, 0.5, recs.size)
+    return PixelMap(recs, counts, offsets)
+
+
+@pytest.mark.parametrize("enc,rows", [("runs", 8), ("runs", 16), ("runs", 32), ("csr", 16)])
+@pytest.mark.parametrize("mode,sem,var", [("floor", "py", False), ("gradient", "py", True), ("bilinear", "omp", False)])
+@pytest.mark.parametrize("n_r,n_eta", [(1, 1), (35, 2), (50, 7), (24, 40)])
+def test_few_frames_equal_the_batch(cuda, enc, rows, mode, sem, var, n_r, n_eta):
+    ny, nz, F = 61, 53, 20
+    rng = np.random.default_rng(n_eta)
+    kw = dict(n_r=n_r, n_eta=n_eta, n_pixels_y=ny, n_pixels_z=nz, mode=mode, semantics=sem, variance=var, bc_y=30.1,
+              bc_z=26.4, device=cuda, encoding=enc, tile_rows=rows)
+    plan = CakePlan(_map(n_r, n_eta, ny, nz, n_r), **kw)
+    if sem == "omp":
+        plan.set_bin_mask(np.arange(n_r * n_eta) % 9 == 4)
+    for dark in (False, True):
+        if dark:
+            plan.set_dark(rng.normal(100, 5, (nz, ny)))
+        for dt in (np.uint8, np.uint16, np.int32, np.uint32, np.int64, np.float32, np.float64):
+            frames = torch.from_numpy(rng.integers(0, 250, (F, nz, ny)).astype(dt)).to(cuda)
+            whole = plan.integrate(frames)
+            for first, n in ((0, 1), (3, 2), (4, 16), (10, 9)) if dt == np.uint16 else ((F - 3, 3),):
+                part = plan.integrate(frames[first:first + n])
+                for x, y in zip(part, whole):
+                    np.testing.assert_array_equal(x.cpu().numpy(), y[first:first + n].cpu().numpy())
+            only, _, _ = plan.integrate(frames[5:6], lineouts=sem == "omp")
+            np.testing.assert_array_equal(only[0].cpu().numpy(), whole[0][5].cpu().numpy())
+    assert plan.status() == 0

@@ -444,12 +444,14 @@ struct Plan {
   int n_sms = 0;
   int mma_stages = 8, mma_producers = 6;   // pipeline of the MMA kernel (mi_plan_set_mma_pipeline)
 
-  // few frames of the run and CSR encodings (mi_one.cu): terms slice by slice
+  // few frames of the run, CSR and MMA encodings (mi_one.cu): terms slice by slice
   PlainLayout one;
   int32_t *d_one_cnt = nullptr;
   int64_t *d_one_ptr = nullptr;
-  uint2 *d_one_terms = nullptr;    // {pixel | kOneEnd, weight}
+  uint2 *d_one_terms = nullptr;    // {pixel | kOneEnd, weight (MMA encoding: q)}
   double *d_one_scale = nullptr;   // per bin
+  int32_t *d_one_tile = nullptr;   // MMA encoding: tile of each bin (its factor and dark term)
+  bool one_res_in_xc = false;      // the bin results live in d_xc
   double *d_one_res = nullptr;     // bin results of kOneChunk frames, for the lineouts
 
   // pixel-major staging (run encoding with 64-frame groups)
@@ -493,8 +495,10 @@ int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t st
 // Run kernel / this, us: 16 frames 311 / 110 (1024^2, 495 x 45), 975 / 369 (2048^2, 990 x 72), 1101 /
 // 640 (2048^2, 1980 x 180 gradient), 1621 / 1114 (2880^2, 3960 x 360 gradient); 32 frames 318 / 218,
 // 996 / 765, 1131 / 1241, 1675 / 2201.  CSR kernel / this, 16 frames: 139 / 91, 703 / 291, 1036 / 413,
-// 1807 / 784.
-constexpr int kOneFrames = 16;
+// 1807 / 784.  MMA kernel / this: 8 frames 147 / 66, 149 / 80, 513 / 226, 581 / 312, 804 / 452 (1024^2
+// floor and bilinear, 2048^2 floor and gradient, 2880^2); 16 frames 148 / 124, 151 / 155, 519 / 451,
+// 589 / 616, 816 / 898.
+constexpr int kOneFrames = 16, kOneFramesMma = 12;
 constexpr int kOneChunk = 8;     // frames whose bin results are held for the lineouts
 int build_one(Plan *p, size_t *acct);
 int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,

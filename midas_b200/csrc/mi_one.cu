@@ -1,4 +1,4 @@
-// mi_one.cu -- kernel (b) for a few frames: the run and CSR encodings' sums, thread per bin.
+// mi_one.cu -- kernel (b) for a few frames: the run, CSR and MMA encodings' sums, thread per bin.
 //
 // The batched kernels' lanes are frames: one frame leaves 31 of 32 lanes idle, and their cost is
 // per pass over the map.  Here a lane is a bin.  A bin's terms {pixel, weight} are the ones of
@@ -8,12 +8,16 @@
 // pixel that is not finite reaches the bins whose terms hold it; the run kernel's zero weights
 // spread it to other bins of the same strip.)
 //
+// MMA plans: the terms carry the fixed-point weights, the sums are exact 64-bit integers and are
+// scaled as the tensor-core kernel's epilogue scales them: the same bits again.
+//
 // Layout: slices of 32 neighbouring bins as in the plain path (PlainLayout): step k holds term k
 // of each bin that has one, side by side, nothing padded, 8 B a term.  It is made on the device
 // from the tile blobs when the plan is.
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "mi_internal.h"
@@ -99,6 +103,7 @@ struct OneBuild {
   const int64_t *slice_ptr;
   uint2 *terms;
   double *scale;
+  const int32_t *xc_pix;    // MMA encoding: pixel of a compact index
   int n_tiles, enc, G, L;
 };
 
@@ -164,6 +169,85 @@ __global__ void k_one_fill(OneBuild a) {
   }
 }
 
+// MMA encoding: a tile's words, each up to four terms of one bin.  The sums are exact integers, so
+// the order of a bin's terms is free: a term takes the next place of its bin.
+__device__ __forceinline__ int64_t mma_bin(const PlainLayout &g, const MmaHdr &h, int n) {
+  const int row = n / kMmaCols, col = n % kMmaCols;
+  return row < h.n_rows && col < h.n_cols ? (int64_t)(h.r0 + row) * g.n_eta + h.e0 + col : -1;
+}
+// slice and lane of a bin (the inverse of plain_bin)
+__device__ __forceinline__ int64_t plain_slot(const PlainLayout &g, int64_t b) {
+  const int64_t per_row = (g.n_eta + (1 << g.ee) - 1) >> g.ee, r = b / g.n_eta, e = b % g.n_eta;
+  const int rr = 32 >> g.ee;
+  return ((r / rr) * per_row + (e >> g.ee)) * 32 + (r % rr << g.ee) + (e & ((1 << g.ee) - 1));
+}
+
+template <bool FILL>
+__global__ void __launch_bounds__(128) k_one_mma(OneBuild a) {
+  __shared__ int32_t s_n[kMmaN];
+  const uint8_t *blob = a.blobs + a.tiles[blockIdx.x].off;
+  const MmaHdr h = *(const MmaHdr *)blob;
+  const MmaBlob B = mma_blob_layout(h.n_k, h.n_runs, h.n_terms);
+  const uint2 *runs = (const uint2 *)(blob + B.runs);
+  const uint32_t *rptr = (const uint32_t *)(blob + B.run_ptr), *sp = (const uint32_t *)(blob + B.step_ptr);
+  const uint4 *wpl = (const uint4 *)(blob + B.wpl);
+  const uint16_t *widx = (const uint16_t *)(blob + B.widx);
+  for (int n = threadIdx.x; n < kMmaN; n += blockDim.x) {
+    s_n[n] = 0;
+    const int64_t b = mma_bin(a.g, h, n);
+    if (!FILL && b >= 0) a.tile_of_bin[b] = (int)blockIdx.x;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < h.n_terms; t += blockDim.x) {
+    const int n = widx[t] >> 3;
+    const uint4 wv = wpl[t];
+    int lo = 0, hi = h.n_k - 1;          // the word's K step
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (sp[mid] <= (uint32_t)t) lo = mid;
+      else hi = mid - 1;
+    }
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t dg = ((wv.x >> (8 * c)) & 0xFFu) | (((wv.y >> (8 * c)) & 0xFFu) << 8) |
+                          (((wv.z >> (8 * c)) & 0xFFu) << 16) | (((wv.w >> (8 * c)) & 0xFFu) << 24);
+      if (dg == 0u) continue;
+      const int k = atomicAdd(&s_n[n], 1);
+      if constexpr (FILL) {
+        const uint32_t kk = (widx[t] & 7u) * 4u + (uint32_t)c;   // K slot; its pixel: the run that covers it
+        uint32_t px = 0;
+        for (uint32_t r = rptr[lo]; r < rptr[lo + 1]; ++r) {
+          const uint32_t k0 = runs[r].y & 0xFFu, len = runs[r].y >> 8;
+          if (kk >= k0 && kk < k0 + len) px = (uint32_t)a.xc_pix[runs[r].x + (kk - k0)];
+        }
+        const int64_t slot = plain_slot(a.g, mma_bin(a.g, h, n)), s = slot >> 5;
+        const int lane = (int)(slot & 31);
+        int64_t o = a.slice_ptr[s];
+        for (int l = 0; l < 32; ++l) {
+          const int m = a.cnt[s * 32 + l];
+          o += min(m, k) + (l < lane && m > k ? 1 : 0);
+        }
+        a.terms[o] = make_uint2(px, (uint32_t)(int32_t)mma_digits_value(dg));
+      }
+    }
+  }
+  if constexpr (!FILL) {
+    __syncthreads();
+    for (int n = threadIdx.x; n < kMmaN; n += blockDim.x) {
+      const int64_t b = mma_bin(a.g, h, n);
+      if (b >= 0) a.cnt[plain_slot(a.g, b)] = s_n[n];
+    }
+  }
+}
+
+__global__ void k_one_slices(OneBuild a) {
+  const int lane = threadIdx.x & 31;
+  const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (s >= a.g.n_slices) return;
+  int64_t t = a.cnt[s * 32 + lane];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) a.slice_n[s] = t;
+}
+
 struct OneArgs {
   PlainLayout g;
   const uint2 *terms;
@@ -177,6 +261,9 @@ struct OneArgs {
   double *res;              // [F][n_bins] for the lineouts, or null
   int64_t n_bins;
   int F, round_res;         // round_res: the lineouts take the rounded bin results (CSR encoding)
+  const int32_t *tile_of_bin;   // MMA encoding: where a bin's factor and dark term are
+  const TileRef *tiles;
+  const uint8_t *blobs;
 };
 
 // NF frames per pass over the map, U terms in flight per lane and as many fetched ahead.  Bounded
@@ -184,8 +271,10 @@ struct OneArgs {
 // at few bins by their latency.  One frame, cake only, where the run kernel took 298, 936, 1038 and
 // 1525 us: 33, 48, 67 and 112 us (1024^2, 495 x 45; 2048^2, 990 x 72; 1980 x 180 gradient; 2880^2,
 // 3960 x 360 gradient, 308 MB of terms).
-template <typename T, int NF, int U>
+// INT (MMA encoding): integer weights, exact integer sums, the kernel's scaling.
+template <typename T, int NF, int U, bool INT>
 __global__ void __launch_bounds__(128) k_one(OneArgs a) {
+  using Acc = typename std::conditional<INT, long long, double>::type;
   const int lane = threadIdx.x & 31;
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= a.g.n_slices) return;
@@ -198,11 +287,13 @@ __global__ void __launch_bounds__(128) k_one(OneArgs a) {
   int64_t at = first;
   const int f0 = (int)blockIdx.y * NF;
   const T *img[NF];
-  double acc[NF], tot[NF];
+  Acc acc[NF];
+  double tot[NF];
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     img[q] = (const T *)a.frames + (int64_t)min(f0 + q, a.F - 1) * a.stride;
-    acc[q] = tot[q] = 0.0;
+    acc[q] = 0;
+    tot[q] = 0.0;
   }
   uint2 t[U];
   if (n_max > 0) plain_load<uint2, U>(a.terms, first, 0, n, lane, at, t);
@@ -216,16 +307,22 @@ __global__ void __launch_bounds__(128) k_one(OneArgs a) {
       const uint32_t p = t[u].x & ~kOneEnd;
 #pragma unroll
       for (int q = 0; q < NF; ++q) raw[u][q] = __ldg(img[q] + p);
-      d[u] = a.dark ? __ldg(a.dark + p) : 0.0f;
+      d[u] = !INT && a.dark ? __ldg(a.dark + p) : 0.0f;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const double w = (double)__uint_as_float(t[u].y);
       const bool in = k + u < n;
+      if constexpr (INT) {
+        const long long w = in ? (long long)(int32_t)t[u].y : 0;
+#pragma unroll
+        for (int q = 0; q < NF; ++q) acc[q] += w * (long long)(int32_t)raw[u][q];
+        continue;
+      }
+      const double w = (double)__uint_as_float(t[u].y);
 #pragma unroll
       for (int q = 0; q < NF; ++q) {
-        const double x = fma(w, (double)((float)raw[u][q] - d[u]), acc[q]);
-        acc[q] = in ? x : acc[q];
+        const double x = fma(w, (double)((float)raw[u][q] - d[u]), (double)acc[q]);
+        acc[q] = in ? (Acc)x : acc[q];
       }
       if (in && (t[u].x & kOneEnd)) {
 #pragma unroll
@@ -239,11 +336,22 @@ __global__ void __launch_bounds__(128) k_one(OneArgs a) {
     for (int u = 0; u < U; ++u) t[u] = tn[u];
   }
   if (b < 0) return;
-  const double sc = a.scale[b];
+  double sc, dk = 0.0;
+  if constexpr (INT) {
+    const uint8_t *blob = a.blobs + a.tiles[a.tile_of_bin[b]].off;
+    const MmaHdr h = *(const MmaHdr *)blob;
+    const int m = ((int)(b / a.g.n_eta) - h.r0) * kMmaCols + (int)(b % a.g.n_eta) - h.e0;
+    sc = ((const double *)(blob + kMmaBinsOff))[m];
+    dk = ((const double *)(blob + kMmaBinsOff))[kMmaN + m];
+  } else {
+    sc = a.scale[b];
+  }
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     if (f0 + q >= a.F) break;
-    const double o = (tot[q] + acc[q]) * sc;   // one of the two is zero
+    double o;
+    if constexpr (INT) o = fma(sc, __ll2double_rn(acc[q]), -dk);
+    else o = (tot[q] + (double)acc[q]) * sc;   // one of the two is zero
     const int64_t at_bin = (int64_t)(f0 + q) * a.n_bins + b;
     if (a.cake) a.cake[at_bin] = (float)o;
     if (a.res) a.res[at_bin] = a.round_res ? (double)(float)o : o;
@@ -264,6 +372,23 @@ __global__ void k_one_partials(const WorkItem *items, int n_items, const TileRef
   double paw = 0.0, psm = 0.0;
   for (int k = it.tile_begin; k < it.tile_end; ++k) {
     const uint8_t *blob = blobs + tiles[k].off;
+    if (enc == MI_ENC_MMA) {
+      const MmaHdr h = *(const MmaHdr *)blob;
+      if (r < h.r0 || r >= h.r0 + h.n_rows) continue;
+      const float *lw = (const float *)(blob + kMmaBinsOff + 16 * kMmaN) + (r - h.r0) * kMmaCols;
+      const double *v = res + f * n_bins + (int64_t)r * n_eta + h.e0;
+      double rw[kMmaCols], rs[kMmaCols];
+#pragma unroll
+      for (int c = 0; c < kMmaCols; ++c) {
+        const double o = c < h.n_cols ? v[c] : 0.0;
+        const float l = lw[c];
+        rw[c] = o * (double)l;
+        rs[c] = (l > 0.0f) ? o : 0.0;
+      }
+      paw += (rw[0] + rw[1]) + (rw[2] + rw[3]);
+      psm += (rs[0] + rs[1]) + (rs[2] + rs[3]);
+      continue;
+    }
     const TileHdr h = *(const TileHdr *)blob;
     if (r < h.r0 || r >= h.r0 + h.n_rows) continue;
     uint32_t o0, o1, o_lw, o3, o4, o5, o6;
@@ -289,7 +414,8 @@ __global__ void k_one_partials(const WorkItem *items, int n_items, const TileRef
 int build_one(Plan *p, size_t *acct) {
   p->one = plain_layout(p->n_r, p->n_eta);
   const PlainLayout &g = p->one;
-  if (p->n_tiles == 0 || (p->encoding != MI_ENC_RUNS && p->encoding != MI_ENC_CSR)) return MI_OK;
+  if (p->n_tiles == 0 || p->encoding == MI_ENC_MMAD) return MI_OK;
+  const bool mma = p->encoding == MI_ENC_MMA;
   cudaStream_t st = nullptr;
   MI_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   std::vector<void *> tmp;
@@ -311,18 +437,35 @@ int build_one(Plan *p, size_t *acct) {
     a.enc = p->encoding;
     a.G = p->run_g;
     a.L = p->run_l;
-    MI_CUDA(temp((void **)&a.tile_of_bin, sizeof(int32_t) * p->n_bins));
+    if (mma) {
+      MI_CUDA(keep((void **)&p->d_one_tile, sizeof(int32_t) * p->n_bins));
+      a.tile_of_bin = p->d_one_tile;
+    } else {
+      MI_CUDA(temp((void **)&a.tile_of_bin, sizeof(int32_t) * p->n_bins));
+    }
+    a.xc_pix = p->d_xc_pix;
     MI_CUDA(temp((void **)&a.slice_n, sizeof(int64_t) * g.n_slices));
     MI_CUDA(keep((void **)&p->d_one_cnt, sizeof(int32_t) * 32 * g.n_slices));
     MI_CUDA(keep((void **)&p->d_one_ptr, sizeof(int64_t) * g.n_slices));
-    MI_CUDA(keep((void **)&p->d_one_scale, sizeof(double) * p->n_bins));
-    MI_CUDA(keep((void **)&p->d_one_res, sizeof(double) * p->n_bins * kOneChunk));
+    if (!mma) MI_CUDA(keep((void **)&p->d_one_scale, sizeof(double) * p->n_bins));
+    // the bin results live in the pixel-major buffer, which this path leaves alone, where it is
+    // large enough
+    const size_t res = sizeof(double) * p->n_bins * kOneChunk;
+    p->one_res_in_xc = p->n_xc * kXcRowBytes >= (int64_t)res;
+    if (!p->one_res_in_xc) MI_CUDA(keep((void **)&p->d_one_res, res));
     a.cnt = p->d_one_cnt;
     a.scale = p->d_one_scale;
     const unsigned blocks = (unsigned)((g.n_slices * 32 + 127) / 128);
-    k_one_tiles<<<(unsigned)p->n_tiles, 128, 0, st>>>(a);
-    MI_CUDA(cudaGetLastError());
-    k_one_count<<<blocks, 128, 0, st>>>(a);
+    if (mma) {
+      MI_CUDA(cudaMemsetAsync(p->d_one_cnt, 0, sizeof(int32_t) * 32 * g.n_slices, st));
+      k_one_mma<false><<<(unsigned)p->n_tiles, 128, 0, st>>>(a);
+      MI_CUDA(cudaGetLastError());
+      k_one_slices<<<blocks, 128, 0, st>>>(a);
+    } else {
+      k_one_tiles<<<(unsigned)p->n_tiles, 128, 0, st>>>(a);
+      MI_CUDA(cudaGetLastError());
+      k_one_count<<<blocks, 128, 0, st>>>(a);
+    }
     MI_CUDA(cudaGetLastError());
     std::vector<int64_t> n(g.n_slices);
     MI_CUDA(cudaMemcpyAsync(n.data(), a.slice_n, sizeof(int64_t) * g.n_slices, cudaMemcpyDeviceToHost, st));
@@ -337,7 +480,8 @@ int build_one(Plan *p, size_t *acct) {
     MI_CUDA(keep((void **)&p->d_one_terms, sizeof(uint2) * total));
     a.slice_ptr = p->d_one_ptr;
     a.terms = p->d_one_terms;
-    k_one_fill<<<blocks, 128, 0, st>>>(a);
+    if (mma) k_one_mma<true><<<(unsigned)p->n_tiles, 128, 0, st>>>(a);
+    else k_one_fill<<<blocks, 128, 0, st>>>(a);
     MI_CUDA(cudaGetLastError());
     MI_CUDA(cudaStreamSynchronize(st));
     return MI_OK;
@@ -349,17 +493,17 @@ int build_one(Plan *p, size_t *acct) {
   return rc;
 }
 
-template <typename T>
+template <typename T, bool INT>
 static int launch_one_t(Plan *p, const OneArgs &a, cudaStream_t s) {
   const unsigned bx = (unsigned)((p->one.n_slices * 32 + 127) / 128);
   const bool deep = p->one.n_slices < kPlainDeep * (int64_t)std::max(p->n_sms, 1);
   if (a.F == 1) {
-    if (deep) k_one<T, 1, 16><<<dim3(bx, 1), 128, 0, s>>>(a);
-    else k_one<T, 1, 8><<<dim3(bx, 1), 128, 0, s>>>(a);
+    if (deep) k_one<T, 1, 16, INT><<<dim3(bx, 1), 128, 0, s>>>(a);
+    else k_one<T, 1, 8, INT><<<dim3(bx, 1), 128, 0, s>>>(a);
   } else if (a.F == 2) {
-    k_one<T, 2, 8><<<dim3(bx, 1), 128, 0, s>>>(a);
+    k_one<T, 2, 8, INT><<<dim3(bx, 1), 128, 0, s>>>(a);
   } else {
-    k_one<T, 4, 4><<<dim3(bx, (unsigned)((a.F + 3) / 4)), 128, 0, s>>>(a);
+    k_one<T, 4, 4, INT><<<dim3(bx, (unsigned)((a.F + 3) / 4)), 128, 0, s>>>(a);
   }
   MI_CUDA(cudaGetLastError());
   return MI_OK;
@@ -377,26 +521,32 @@ static int launch_one_chunk(Plan *p, const void *frames, int dtype, int F, int64
   a.stride = stride;
   a.dark = p->has_dark ? p->d_dark : nullptr;
   a.cake = cake;
-  a.res = want_lo ? p->d_one_res : nullptr;
+  double *res = p->one_res_in_xc ? (double *)p->d_xc : p->d_one_res;
+  a.res = want_lo ? res : nullptr;
   a.n_bins = p->n_bins;
   a.F = F;
   a.round_res = p->encoding == MI_ENC_CSR;
+  a.tile_of_bin = p->d_one_tile;
+  a.tiles = p->d_tiles;
+  a.blobs = p->d_blobs;
   int rc = MI_OK;
-  switch (dtype) {
-    case MI_DT_U8: rc = launch_one_t<uint8_t>(p, a, s); break;
-    case MI_DT_U16: rc = launch_one_t<uint16_t>(p, a, s); break;
-    case MI_DT_U32: rc = launch_one_t<uint32_t>(p, a, s); break;
-    case MI_DT_I64: rc = launch_one_t<int64_t>(p, a, s); break;
-    case MI_DT_F32: rc = launch_one_t<float>(p, a, s); break;
-    case MI_DT_F64: rc = launch_one_t<double>(p, a, s); break;
-    case MI_DT_I32: rc = launch_one_t<int32_t>(p, a, s); break;
+  if (p->encoding == MI_ENC_MMA) {
+    rc = dtype == MI_DT_U8 ? launch_one_t<uint8_t, true>(p, a, s) : launch_one_t<uint16_t, true>(p, a, s);
+  } else switch (dtype) {
+    case MI_DT_U8: rc = launch_one_t<uint8_t, false>(p, a, s); break;
+    case MI_DT_U16: rc = launch_one_t<uint16_t, false>(p, a, s); break;
+    case MI_DT_U32: rc = launch_one_t<uint32_t, false>(p, a, s); break;
+    case MI_DT_I64: rc = launch_one_t<int64_t, false>(p, a, s); break;
+    case MI_DT_F32: rc = launch_one_t<float, false>(p, a, s); break;
+    case MI_DT_F64: rc = launch_one_t<double, false>(p, a, s); break;
+    case MI_DT_I32: rc = launch_one_t<int32_t, false>(p, a, s); break;
     default: return set_error(MI_E_ARG, "unknown dtype %d", dtype);
   }
   if (rc || !want_lo) return rc;
-  const int rows = p->lim.rows;
+  const int rows = p->encoding == MI_ENC_MMA ? kMmaRows : p->lim.rows;
   const int64_t n = (int64_t)p->n_items * rows;
   k_one_partials<<<dim3((unsigned)((n + 127) / 128), (unsigned)F), 128, 0, s>>>(
-      p->d_items, p->n_items, p->d_tiles, p->d_blobs, p->encoding, p->run_g, p->run_l, rows, p->d_one_res, p->n_bins,
+      p->d_items, p->n_items, p->d_tiles, p->d_blobs, p->encoding, p->run_g, p->run_l, rows, res, p->n_bins,
       p->n_r, p->n_eta, p->n_slots, partial);
   MI_CUDA(cudaGetLastError());
   return MI_OK;

@@ -573,7 +573,8 @@ static int free_plan_mem(Plan *p) {
                   p->d_plain_t4, p->d_area_gs, p->d_area_in, p->d_plain_img,
                   p->d_ctr, p->d_span_lo, p->d_row_off, p->d_xchunks, p->d_xc,
                   p->d_xc_pix, p->d_nan_bins, p->d_upload,
-                  p->d_one_cnt, p->d_one_ptr, p->d_one_terms, p->d_one_scale, p->d_one_res};
+                  p->d_one_cnt, p->d_one_ptr, p->d_one_terms, p->d_one_scale, p->d_one_tile,
+                  p->d_one_res};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   return MI_OK;

@@ -50,3 +50,24 @@ def test_few_frames_equal_the_batch(cuda, enc, rows, mode, sem, var, n_r, n_eta)
             only, _, _ = plan.integrate(frames[5:6], lineouts=sem == "omp")
             np.testing.assert_array_equal(only[0].cpu().numpy(), whole[0][5].cpu().numpy())
     assert plan.status() == 0
+
+
+@pytest.mark.parametrize("mode,sem,var", [("floor", "py", False), ("gradient", "py", True), ("bilinear", "ic", False)])
+@pytest.mark.parametrize("n_r,n_eta", [(1, 1), (13, 2), (50, 7), (24, 40)])
+def test_few_frames_equal_the_batch_on_the_tensor_cores(cuda, mode, sem, var, n_r, n_eta):
+    """MMA plans: 1 to 12 frames by the lane-per-bin kernel, 20 by the tensor cores; the first
+    call after a dark is set or cleared follows it."""
+    ny, nz, F = 61, 53, 20
+    rng = np.random.default_rng(n_eta)
+    plan = CakePlan(_map(n_r, n_eta, ny, nz, n_r), n_r=n_r, n_eta=n_eta, n_pixels_y=ny, n_pixels_z=nz, mode=mode,
+                    semantics=sem, variance=var, bc_y=30.1, bc_z=26.4, device=cuda, encoding="mma")
+    for dark in (None, rng.normal(100, 5, (nz, ny)), None):
+        plan.set_dark(dark)
+        for dt, top in ((np.uint8, 256), (np.uint16, 65536)):
+            frames = torch.from_numpy(rng.integers(0, top, (F, nz, ny)).astype(dt)).to(cuda)
+            parts = [(f, n, plan.integrate(frames[f:f + n])) for f, n in ((0, 1), (3, 2), (4, 12), (10, 9))]
+            whole = plan.integrate(frames)
+            for f, n, part in parts:
+                for x, y in zip(part, whole):
+                    np.testing.assert_array_equal(x.cpu().numpy(), y[f:f + n].cpu().numpy())
+    assert plan.status() == 0

@@ -366,7 +366,10 @@ int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t st
   if (!a.want_cake && !a.want_lo) return MI_OK;
   int rc = MI_OK;
   const bool mma = p->encoding == MI_ENC_MMA, u16 = dtype == MI_DT_U16 || dtype == MI_DT_U8;
-  if (p->d_one_terms && n_frames <= (mma ? kOneFramesMma : kOneFrames) && (!mma || u16)) {
+  if (n_frames >= kOnePmMin && (!u16 || n_frames <= kOnePmU16) && one_pm_fits(p, a.want_lo)) {
+    // run plans: eight frames of a pixel side by side, a lane per bin (mi_one.cu)
+    rc = launch_one_pm(p, &frames, &dtype, &stride, 0, n_frames, cake, partial, a.want_lo, s);
+  } else if (p->d_one_terms && n_frames <= (mma ? kOneFramesMma : kOneFrames) && (!mma || u16)) {
     // few frames: a lane per bin, the same sums (mi_one.cu)
     rc = launch_one(p, frames, dtype, n_frames, stride, cake, partial, a.want_lo, s);
   } else if (p->encoding == MI_ENC_MMA) {

@@ -500,7 +500,18 @@ int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t st
 // 589 / 616, 816 / 898.
 constexpr int kOneFrames = 16, kOneFramesMma = 12;
 constexpr int kOneChunk = 8;     // frames whose bin results are held for the lineouts
+// Run plans from kOnePmMin frames on: eight frames of a pixel side by side (launch_one_pm), for 8/16-bit
+// frames up to kOnePmU16.  Lane per bin over frames / this, us: 4 frames 110 / 143 (1475 x 1679 i32), 166
+// / 179 (2048^2, 990 x 72), 8 frames 156 / 144, 214 / 177, 16 frames 319 / 184, 427 / 274.  Run kernel /
+// this: i32, 64 frames 1146 / 643, 1957 / 985, 2156 / 1586 (1980 x 180 gradient), 1151 / 1147 (1440^2,
+// 3960 x 360 gradient); u16, 32 frames 1007 / 488, 1136 / 786, 628 / 572; 48 frames 1024 / 762, 1163 /
+// 1189, 652 / 855.
+constexpr int kOnePmMin = 5, kOnePmU16 = 32;
 int build_one(Plan *p, size_t *acct);
+bool one_pm_fits(const Plan *p, bool want_lo);
+// frames [first, first + F) of every panel; cake and partial are those of the first
+int launch_one_pm(Plan *p, const void *const *frames, const int *dtypes, const int64_t *strides, int first, int F,
+                  float *cake, double *partial, bool want_lo, cudaStream_t s);
 int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
                bool want_lo, cudaStream_t s);
 int launch_runs(Plan *p, const void *frames, int dtype, int n_frames, int64_t stride, float *cake, double *partial,

@@ -24,6 +24,8 @@
 
 namespace mi {
 
+constexpr int kPmFrames = 8;                // frames of a pixel side by side
+static_assert(kOneChunk <= kPmFrames, "the bin results hold eight frames a bin");
 constexpr uint32_t kOneEnd = 0x80000000u;   // the term ends a unit partial
 
 // The terms of one bin in summing order.  Run encoding: the units of the bin's strip, records in
@@ -104,6 +106,8 @@ struct OneBuild {
   uint2 *terms;
   double *scale;
   const int32_t *xc_pix;    // MMA encoding: pixel of a compact index
+  const int32_t *span_lo, *row_off;   // panel plans: the terms name compact indices
+  int ny;
   int n_tiles, enc, G, L;
 };
 
@@ -162,6 +166,10 @@ __global__ void k_one_fill(OneBuild a) {
   for (int k = 0; __any_sync(0xffffffffu, k < n); ++k) {
     const int64_t o = plain_step(k < n, lane, at);
     if (k >= n) continue;
+    if (a.row_off) {
+      const int z = (int)(pix / (uint32_t)a.ny);
+      pix = (uint32_t)(a.row_off[z] + (int)(pix - (uint32_t)z * (uint32_t)a.ny) - a.span_lo[z]);
+    }
     uint2 t = make_uint2(pix, __float_as_uint(w));
     more = it.next(&pix, &w, &first);
     if (a.enc == MI_ENC_RUNS && (!more || first)) t.x |= kOneEnd;
@@ -258,7 +266,7 @@ struct OneArgs {
   int64_t stride;
   const float *dark;        // null: none
   float *cake;              // [F][n_bins] or null
-  double *res;              // [F][n_bins] for the lineouts, or null
+  double *res;              // [F / 8][n_bins][8] for the lineouts, or null
   int64_t n_bins;
   int F, round_res;         // round_res: the lineouts take the rounded bin results (CSR encoding)
   const int32_t *tile_of_bin;   // MMA encoding: where a bin's factor and dark term are
@@ -354,21 +362,116 @@ __global__ void __launch_bounds__(128) k_one(OneArgs a) {
     else o = (tot[q] + (double)acc[q]) * sc;   // one of the two is zero
     const int64_t at_bin = (int64_t)(f0 + q) * a.n_bins + b;
     if (a.cake) a.cake[at_bin] = (float)o;
-    if (a.res) a.res[at_bin] = a.round_res ? (double)(float)o : o;
+    if (a.res) a.res[b * kPmFrames + f0 + q] = a.round_res ? (double)(float)o : o;   // F <= kOneChunk = 8
+  }
+}
+
+// ---- many frames, eight to a 32-byte sector
+//
+// Beyond a few frames the gathers bound k_one: a lane's pixels lie in different lines whatever a
+// line brings.  Here eight frames of a pixel lie side by side as fp32 minus the dark (one
+// sector), so a gather brings eight values and a term is read once for them.  Bounded by the
+// sectors from L2 (1475 x 1679 int32, 790 x 72 bins, 50 frames: 317 us for 29 M gathers, 2.9 TB/s) and by
+// the staging pass's bytes (150 us, 6 TB/s).  50 such frames with lineouts took 1078 us through the
+// 64-frame rows and the run kernel, 800 through k_one; 534 here.
+//
+// k_pm writes them: a thread per pixel of a span, eight coalesced loads, one 32-byte store.
+template <typename T>
+__global__ void __launch_bounds__(256) k_pm(const T *__restrict__ frames, int64_t stride, int F, int ny, int z_off,
+                                            int ny_v, const float *__restrict__ dark,
+                                            const XcChunk *__restrict__ chunks, float *__restrict__ pm, int64_t n_px,
+                                            int compact) {
+  const XcChunk ch = chunks[blockIdx.x];
+  if ((int)threadIdx.x >= ch.n) return;
+  const int f0 = (int)blockIdx.y * kPmFrames;
+  const int64_t o = (int64_t)(ch.z - z_off) * ny + ch.y0 + threadIdx.x;
+  const int64_t v = (int64_t)ch.z * ny_v + ch.y0 + threadIdx.x;
+  T raw[kPmFrames];
+#pragma unroll
+  for (int q = 0; q < kPmFrames; ++q) raw[q] = f0 + q < F ? __ldg(frames + (int64_t)(f0 + q) * stride + o) : (T)0;
+  const float d = __ldg(dark + v);
+  float x[kPmFrames];
+#pragma unroll
+  for (int q = 0; q < kPmFrames; ++q) x[q] = f0 + q < F ? (float)raw[q] - d : 0.0f;
+  const int64_t at = compact ? (int64_t)ch.c0 + threadIdx.x : v;
+  float4 *dst = (float4 *)(pm + ((int64_t)blockIdx.y * n_px + at) * kPmFrames);
+  dst[0] = make_float4(x[0], x[1], x[2], x[3]);
+  dst[1] = make_float4(x[4], x[5], x[6], x[7]);
+}
+
+template <int U>
+__global__ void __launch_bounds__(128) k_one_pm(OneArgs a, const float *pm, int64_t n_px) {
+  const int lane = threadIdx.x & 31;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (i >= a.g.n_slices) return;
+  const int64_t s = a.g.n_slices - 1 - i;
+  const int64_t b = plain_bin(a.g, s, lane);
+  const int n = a.cnt[s * 32 + lane];
+  int n_max = n;
+  for (int o = 16; o > 0; o >>= 1) n_max = max(n_max, __shfl_xor_sync(0xffffffffu, n_max, o));
+  const int64_t first = a.slice_ptr[s];
+  int64_t at = first;
+  const float4 *src = (const float4 *)(pm + (int64_t)blockIdx.y * n_px * kPmFrames);
+  double acc[kPmFrames], tot[kPmFrames];
+#pragma unroll
+  for (int q = 0; q < kPmFrames; ++q) acc[q] = tot[q] = 0.0;
+  uint2 t[U];
+  if (n_max > 0) plain_load<uint2, U>(a.terms, first, 0, n, lane, at, t);
+  for (int k = 0; k < n_max; k += U) {
+    uint2 tn[U];
+    if (k + U < n_max) plain_load<uint2, U>(a.terms, first, k + U, n, lane, at, tn);
+    float4 x[U][2];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float4 *r = src + 2 * (int64_t)(t[u].x & ~kOneEnd);
+      x[u][0] = __ldg(r);
+      x[u][1] = __ldg(r + 1);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (k + u >= n) break;
+      const double w = (double)__uint_as_float(t[u].y);
+      const float v[kPmFrames] = {x[u][0].x, x[u][0].y, x[u][0].z, x[u][0].w,
+                                  x[u][1].x, x[u][1].y, x[u][1].z, x[u][1].w};
+#pragma unroll
+      for (int q = 0; q < kPmFrames; ++q) acc[q] = fma(w, (double)v[q], acc[q]);
+      if (t[u].x & kOneEnd) {
+#pragma unroll
+        for (int q = 0; q < kPmFrames; ++q) {
+          tot[q] += (double)(float)acc[q];
+          acc[q] = 0.0;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) t[u] = tn[u];
+  }
+  if (b < 0) return;
+  const double sc = a.scale[b];
+  const int f0 = (int)blockIdx.y * kPmFrames;
+#pragma unroll
+  for (int q = 0; q < kPmFrames; ++q) {
+    if (f0 + q >= a.F) break;
+    const double o = (tot[q] + acc[q]) * sc;
+    if (a.cake) a.cake[(int64_t)(f0 + q) * a.n_bins + b] = (float)o;
+    if (a.res) a.res[((int64_t)blockIdx.y * a.n_bins + b) * kPmFrames + q] = o;
   }
 }
 
 // Lineout partials of the items' rows from the bin results, in the batched kernels' order: a
-// tile's columns in order, then the tiles.  One thread per (frame, item, row).
+// tile's columns in order, then the tiles.  One thread per (item, row, frame of eight): the eight
+// frames of a bin lie side by side, and share the walk over the tiles.
 __global__ void k_one_partials(const WorkItem *items, int n_items, const TileRef *tiles, const uint8_t *blobs, int enc,
                                int G, int L, int rows, const double *res, int64_t n_bins, int n_r, int n_eta,
-                               int n_slots, double *partial) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)n_items * rows) return;
-  const int64_t f = blockIdx.y;
+                               int n_slots, int F, double *partial) {
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kPmFrames;
+  const int q = threadIdx.x % kPmFrames;
+  const int64_t f = (int64_t)blockIdx.y * kPmFrames + q;
+  if (t >= (int64_t)n_items * rows || f >= F) return;
   const WorkItem it = items[t / rows];
   const int r = it.r0 + (int)(t % rows);
   if (r >= it.r0 + it.n_rows) return;
+  const double *row = res + ((int64_t)blockIdx.y * n_bins + (int64_t)r * n_eta) * kPmFrames + q;
   double paw = 0.0, psm = 0.0;
   for (int k = it.tile_begin; k < it.tile_end; ++k) {
     const uint8_t *blob = blobs + tiles[k].off;
@@ -376,11 +479,10 @@ __global__ void k_one_partials(const WorkItem *items, int n_items, const TileRef
       const MmaHdr h = *(const MmaHdr *)blob;
       if (r < h.r0 || r >= h.r0 + h.n_rows) continue;
       const float *lw = (const float *)(blob + kMmaBinsOff + 16 * kMmaN) + (r - h.r0) * kMmaCols;
-      const double *v = res + f * n_bins + (int64_t)r * n_eta + h.e0;
       double rw[kMmaCols], rs[kMmaCols];
 #pragma unroll
       for (int c = 0; c < kMmaCols; ++c) {
-        const double o = c < h.n_cols ? v[c] : 0.0;
+        const double o = c < h.n_cols ? row[(int64_t)(h.e0 + c) * kPmFrames] : 0.0;
         const float l = lw[c];
         rw[c] = o * (double)l;
         rs[c] = (l > 0.0f) ? o : 0.0;
@@ -395,10 +497,9 @@ __global__ void k_one_partials(const WorkItem *items, int n_items, const TileRef
     if (enc == MI_ENC_RUNS) runs_blob_layout(h.nb, h.n_cols, h.nnz, h.n_u, G, L, &o0, &o1, &o_lw, &o3, &o4, &o5);
     else blob_layout(h.nb, h.nnz, h.n_u, &o0, &o1, &o_lw, &o3, &o4, &o5, &o6);
     const float *lw = (const float *)(blob + o_lw) + (r - h.r0) * h.n_cols;
-    const double *v = res + f * n_bins + (int64_t)r * n_eta + h.e0;
     double saw = 0.0, ssm = 0.0;
     for (int c = 0; c < h.n_cols; ++c) {
-      const double o = v[c];
+      const double o = row[(int64_t)(h.e0 + c) * kPmFrames];
       const float l = lw[c];
       saw += o * (double)l;
       ssm += (l > 0.0f) ? o : 0.0;
@@ -409,6 +510,16 @@ __global__ void k_one_partials(const WorkItem *items, int n_items, const TileRef
   double *dst = partial + ((f * n_r + r) * n_slots + it.slot) * 2;
   dst[0] = paw;
   dst[1] = psm;
+}
+
+static int launch_one_partials(const Plan *p, const double *res, int F, double *partial, cudaStream_t s) {
+  const int rows = p->encoding == MI_ENC_MMA ? kMmaRows : p->lim.rows;
+  const int64_t n = (int64_t)p->n_items * rows * kPmFrames;
+  k_one_partials<<<dim3((unsigned)((n + 127) / 128), (unsigned)((F + kPmFrames - 1) / kPmFrames)), 128, 0, s>>>(
+      p->d_items, p->n_items, p->d_tiles, p->d_blobs, p->encoding, p->run_g, p->run_l, rows, res, p->n_bins, p->n_r,
+      p->n_eta, p->n_slots, F, partial);
+  MI_CUDA(cudaGetLastError());
+  return MI_OK;
 }
 
 int build_one(Plan *p, size_t *acct) {
@@ -444,6 +555,11 @@ int build_one(Plan *p, size_t *acct) {
       MI_CUDA(temp((void **)&a.tile_of_bin, sizeof(int32_t) * p->n_bins));
     }
     a.xc_pix = p->d_xc_pix;
+    if (p->panels.size() > 1) {
+      a.span_lo = p->d_span_lo;
+      a.row_off = p->d_row_off;
+      a.ny = p->ny;
+    }
     MI_CUDA(temp((void **)&a.slice_n, sizeof(int64_t) * g.n_slices));
     MI_CUDA(keep((void **)&p->d_one_cnt, sizeof(int32_t) * 32 * g.n_slices));
     MI_CUDA(keep((void **)&p->d_one_ptr, sizeof(int64_t) * g.n_slices));
@@ -509,26 +625,31 @@ static int launch_one_t(Plan *p, const OneArgs &a, cudaStream_t s) {
   return MI_OK;
 }
 
-static int launch_one_chunk(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
-                            bool want_lo, cudaStream_t s) {
-  OneArgs a;
+static OneArgs one_args(const Plan *p, int F, float *cake, double *res) {
+  OneArgs a{};
   a.g = p->one;
   a.terms = p->d_one_terms;
   a.cnt = p->d_one_cnt;
   a.slice_ptr = p->d_one_ptr;
   a.scale = p->d_one_scale;
-  a.frames = frames;
-  a.stride = stride;
-  a.dark = p->has_dark ? p->d_dark : nullptr;
   a.cake = cake;
-  double *res = p->one_res_in_xc ? (double *)p->d_xc : p->d_one_res;
-  a.res = want_lo ? res : nullptr;
+  a.res = res;
   a.n_bins = p->n_bins;
   a.F = F;
   a.round_res = p->encoding == MI_ENC_CSR;
   a.tile_of_bin = p->d_one_tile;
   a.tiles = p->d_tiles;
   a.blobs = p->d_blobs;
+  return a;
+}
+
+static int launch_one_chunk(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
+                            bool want_lo, cudaStream_t s) {
+  double *res = !want_lo ? nullptr : (p->one_res_in_xc ? (double *)p->d_xc : p->d_one_res);
+  OneArgs a = one_args(p, F, cake, res);
+  a.frames = frames;
+  a.stride = stride;
+  a.dark = p->has_dark ? p->d_dark : nullptr;
   int rc = MI_OK;
   if (p->encoding == MI_ENC_MMA) {
     rc = dtype == MI_DT_U8 ? launch_one_t<uint8_t, true>(p, a, s) : launch_one_t<uint16_t, true>(p, a, s);
@@ -542,14 +663,7 @@ static int launch_one_chunk(Plan *p, const void *frames, int dtype, int F, int64
     case MI_DT_I32: rc = launch_one_t<int32_t, false>(p, a, s); break;
     default: return set_error(MI_E_ARG, "unknown dtype %d", dtype);
   }
-  if (rc || !want_lo) return rc;
-  const int rows = p->encoding == MI_ENC_MMA ? kMmaRows : p->lim.rows;
-  const int64_t n = (int64_t)p->n_items * rows;
-  k_one_partials<<<dim3((unsigned)((n + 127) / 128), (unsigned)F), 128, 0, s>>>(
-      p->d_items, p->n_items, p->d_tiles, p->d_blobs, p->encoding, p->run_g, p->run_l, rows, res, p->n_bins,
-      p->n_r, p->n_eta, p->n_slots, partial);
-  MI_CUDA(cudaGetLastError());
-  return MI_OK;
+  return rc || !want_lo ? rc : launch_one_partials(p, res, F, partial, s);
 }
 
 int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
@@ -561,6 +675,66 @@ int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, fl
                           stride, cake ? cake + (size_t)f0 * p->n_bins : nullptr,
                           partial + (size_t)f0 * p->n_r * p->n_slots * 2, want_lo, s);
   return rc;
+}
+
+// pixels of an eight-frame block: compact indices for panel plans, whose virtual detector is
+// mostly outside the panels' spans, else the detector's
+static int64_t pm_pixels(const Plan *p) { return p->panels.size() > 1 ? p->n_xc : (int64_t)p->ny * p->nz; }
+
+// eight-frame blocks that fit the pixel-major buffer together with their bin results
+static int64_t pm_blocks(const Plan *p, bool want_lo) {
+  const int64_t per = (pm_pixels(p) * 4 + (want_lo ? p->n_bins * 8 : 0)) * kPmFrames;
+  return p->n_xc * kXcRowBytes / per;
+}
+
+bool one_pm_fits(const Plan *p, bool want_lo) {
+  return p->encoding == MI_ENC_RUNS && p->d_one_terms && p->n_xc > 0 && pm_blocks(p, want_lo) >= 1;
+}
+
+template <typename T>
+static void pm_launch(const Plan *p, const Plan::Panel &pn, const void *frames, int F, int64_t stride, float *pm,
+                      cudaStream_t s) {
+  const dim3 grid((unsigned)(pn.chunk_end - pn.chunk_begin), (unsigned)((F + kPmFrames - 1) / kPmFrames));
+  if (grid.x == 0) return;
+  k_pm<T><<<grid, 256, 0, s>>>((const T *)frames, stride, F, pn.ny, pn.z_off, p->ny, p->d_dark,
+                               p->d_xchunks + pn.chunk_begin, pm, pm_pixels(p), p->panels.size() > 1);
+}
+
+int launch_one_pm(Plan *p, const void *const *frames, const int *dtypes, const int64_t *strides, int first, int F,
+                  float *cake, double *partial, bool want_lo, cudaStream_t s) {
+  const int round = (int)std::min<int64_t>(pm_blocks(p, want_lo), kMaxFramesPerLaunch / kPmFrames) * kPmFrames;
+  for (int f0 = 0; f0 < F; f0 += round) {
+    const int nf = std::min(round, F - f0);
+    const int nb = (nf + kPmFrames - 1) / kPmFrames;
+    float *pm = (float *)p->d_xc;
+    double *res = want_lo ? (double *)(pm + (int64_t)nb * pm_pixels(p) * kPmFrames) : nullptr;
+    for (size_t i = 0; i < p->panels.size(); ++i) {
+      const Plan::Panel &pn = p->panels[i];
+      const void *src = (const uint8_t *)frames[i] + (size_t)(first + f0) * strides[i] * dtype_size(dtypes[i]);
+      switch (dtypes[i]) {
+        case MI_DT_U8: pm_launch<uint8_t>(p, pn, src, nf, strides[i], pm, s); break;
+        case MI_DT_U16: pm_launch<uint16_t>(p, pn, src, nf, strides[i], pm, s); break;
+        case MI_DT_U32: pm_launch<uint32_t>(p, pn, src, nf, strides[i], pm, s); break;
+        case MI_DT_I64: pm_launch<int64_t>(p, pn, src, nf, strides[i], pm, s); break;
+        case MI_DT_F32: pm_launch<float>(p, pn, src, nf, strides[i], pm, s); break;
+        case MI_DT_F64: pm_launch<double>(p, pn, src, nf, strides[i], pm, s); break;
+        case MI_DT_I32: pm_launch<int32_t>(p, pn, src, nf, strides[i], pm, s); break;
+        default: return set_error(MI_E_ARG, "unknown dtype %d", dtypes[i]);
+      }
+      MI_CUDA(cudaGetLastError());
+    }
+    const OneArgs a = one_args(p, nf, cake ? cake + (size_t)f0 * p->n_bins : nullptr, res);
+    const dim3 grid((unsigned)((p->one.n_slices * 32 + 127) / 128), (unsigned)nb);
+    // terms in flight per lane as in the plain path's rule
+    if (p->one.n_slices < kPlainDeep * (int64_t)std::max(p->n_sms, 1)) k_one_pm<8><<<grid, 128, 0, s>>>(a, pm, pm_pixels(p));
+    else k_one_pm<4><<<grid, 128, 0, s>>>(a, pm, pm_pixels(p));
+    MI_CUDA(cudaGetLastError());
+    if (want_lo) {
+      const int rc = launch_one_partials(p, res, nf, partial + (size_t)f0 * p->n_r * p->n_slots * 2, s);
+      if (rc) return rc;
+    }
+  }
+  return MI_OK;
 }
 
 }  // namespace mi

@@ -1320,7 +1320,7 @@ static int build_plan(const mi_map_desc &m, const mi_plan_opts &o, Plan *p, Host
 
   if ((rc = upload(&p->d_area_in, csr.area_in.data(), csr.area_in.size(), &acct))) return rc;
   if (!pre && (rc = build_plain(p, m.records, m.nmap, &acct))) return rc;
-  if (p->panels.size() == 1 && (rc = build_one(p, &acct))) return rc;
+  if ((p->panels.size() == 1 || enc == MI_ENC_RUNS) && (rc = build_one(p, &acct))) return rc;
   p->device_bytes = acct;
   return MI_OK;
 }
@@ -1839,7 +1839,11 @@ int mi_integrate_panels(mi_plan *p, const void *const *frames, const int *dtypes
   int rc = MI_OK;
   for (int g0 = 0; g0 < n_frames && rc == MI_OK; g0 += kMaxFramesPerLaunch) {
     const int ng = std::min(kMaxFramesPerLaunch, n_frames - g0);
-    for (int f0 = 0; f0 < ng && rc == MI_OK; f0 += chunk) {
+    const bool pm = one_pm_fits(p, want_lo) && (as_f32 || ng <= kOnePmU16);
+    if (pm)
+      rc = launch_one_pm(p, frames, dtypes, strides, g0, ng, cake ? cake + (size_t)g0 * p->n_bins : nullptr,
+                         p->d_partial, want_lo, s);
+    for (int f0 = pm ? ng : 0; f0 < ng && rc == MI_OK; f0 += chunk) {
       const int nf = std::min(chunk, ng - f0);
       for (int i = 0; i < np && rc == MI_OK; ++i)
         rc = launch_xc(p, i, (const uint8_t *)frames[i] + (size_t)(g0 + f0) * strides[i] * dtype_size(dtypes[i]),

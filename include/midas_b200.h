@@ -473,7 +473,8 @@ typedef struct {
   const double *eta_lo, *eta_hi;/* host, n_eta eta-bin edges (deg)             */
 } mi_binning;
 
-typedef struct mi_map mi_map;   /* built map held on the host                  */
+typedef struct mi_map mi_map;   /* built map (the records of a device build stay on the device
+                                   until mi_map_copy)                           */
 
 /* device >= 0: build on that GPU; device == -1: build on the host cores (OpenMP),
  * same code, used to cross-check the device build.  Entries of a bin are ordered by

@@ -11,7 +11,13 @@
 // FF_HEDM/src/DetectorGeometry.c (dg_pixel_to_REta_corr :95, dg_polygon_area
 // :432, dg_circle_seg_intersect :507, dg_ray_seg_intersect :536,
 // dg_point_in_quad :555, dg_find_unique_vertices :572); the code is written
-// for one thread per pixel with a count pass, a scan and a fill pass.
+// for one thread per pixel: one evaluation of the geometry appends a pixel's records, a scan of
+// the pixels' counts says where they belong, and a stable sort by bin orders them.
+//
+// The geometry's FP64 functions are the cost.  Sines and cosines of the eta edges come from a
+// table, a corner's radius and angle are found once per pixel and not once per bin, a vertex's
+// once, and the candidate eta bins by bisection.  1475 x 1679 pixels, 790 x 72 bins: count and fill
+// pass 5.9 + 6.6 ms, now 4.7 + 0.1 (sample) + 0.1 ms.
 #include <cub/cub.cuh>
 #include <math.h>
 #include <omp.h>
@@ -37,6 +43,8 @@ struct MapGeom {
 struct MapBins {
   int n_r, n_eta;
   const double *rlo, *rhi, *elo, *ehi;
+  const double *slo, *clo, *shi, *chi;   // sin and cos of the eta edges
+  bool sorted;                           // eta edges ascend: candidate bins by bisection
 };
 
 constexpr double kD2R = 0.017453292519943295;  // pi / 180
@@ -130,8 +138,7 @@ MI_HD inline int seg_circle(double y1, double z1, double y2, double z2, double R
   return n;
 }
 
-MI_HD inline bool seg_ray(double y1, double z1, double y2, double z2, double eta, double *hy, double *hz) {
-  const double er = eta * kD2R, ce = cos(er), se = sin(er);
+MI_HD inline bool seg_ray(double y1, double z1, double y2, double z2, double se, double ce, double *hy, double *hz) {
   const double dy = y2 - y1, dz = z2 - z1;
   const double den = dy * ce + dz * se;
   if (fabs(den) < 1e-30) return false;
@@ -209,78 +216,77 @@ MI_HD inline double adj_eta(double et, double emin, double emax) {
   return et;
 }
 
-// overlap area of pixel quad q with bin [rmin,rmax] x [emin,emax]
-MI_HD inline double quad_bin_area(const double q[4][2], double rmin, double rmax, double emin, double emax) {
+// v within [lo, hi] of R, and eta (also a turn away) within [lo, hi], up to kGeomEps
+MI_HD inline bool in_bin(double R, double E, double rmin, double rmax, double emin, double emax) {
+  if (!within(E, emin, emax)) {
+    if (within(E + 360, emin, emax)) E += 360;
+    else if (within(E - 360, emin, emax)) E -= 360;
+  }
+  return within(R, rmin, rmax) && within(E, emin, emax);
+}
+
+// One eta edge pair of a bin with its sines and cosines.
+struct EtaBin {
+  double lo, hi, slo, clo, shi, chi;
+};
+
+// overlap area of pixel quad q (corner radii qR, eta qE) with bin [rmin,rmax] x eta.  Vertices
+// outside the bin are left out as they come; a vertex equal to a later one is dropped.
+MI_HD inline double quad_bin_area(const double q[4][2], const double qR[4], const double qE[4], double rmin,
+                                  double rmax, const EtaBin &eb) {
+  const double emin = eb.lo, emax = eb.hi;
   double ed[kMaxVerts][2];
-  int n = 0;
-  double box[4][2];
-  reta_to_yz(rmin, emin, &box[0][0], &box[0][1]);
-  reta_to_yz(rmin, emax, &box[1][0], &box[1][1]);
-  reta_to_yz(rmax, emin, &box[2][0], &box[2][1]);
-  reta_to_yz(rmax, emax, &box[3][0], &box[3][1]);
-  for (int m = 0; m < 4; ++m) {
-    const double R = sqrt(q[m][0] * q[m][0] + q[m][1] * q[m][1]);
-    const double E = adj_eta(eta_of(q[m][0], q[m][1]), emin, emax);
-    if (R >= rmin && R <= rmax && E >= emin && E <= emax) {
-      ed[n][0] = q[m][0]; ed[n][1] = q[m][1]; ++n;
+  int n = 0, nv = 0;   // vertices found; those inside the bin, in ed
+  auto push = [&](double y, double z, double R, double E) {
+    ++n;
+    if (in_bin(R, E, rmin, rmax, emin, emax)) {
+      ed[nv][0] = y; ed[nv][1] = z; ++nv;
     }
+  };
+  const double box[4][2] = {{-rmin * eb.slo, rmin * eb.clo}, {-rmin * eb.shi, rmin * eb.chi},
+                            {-rmax * eb.slo, rmax * eb.clo}, {-rmax * eb.shi, rmax * eb.chi}};
+  for (int m = 0; m < 4; ++m) {
+    const double R = qR[m];
+    const double E = adj_eta(qE[m], emin, emax);
+    if (R >= rmin && R <= rmax && E >= emin && E <= emax) push(q[m][0], q[m][1], R, qE[m]);
   }
   for (int m = 0; m < 4; ++m)
-    if (in_quad(box[m][0], box[m][1], q)) {
-      ed[n][0] = box[m][0]; ed[n][1] = box[m][1]; ++n;
-    }
+    if (in_quad(box[m][0], box[m][1], q))
+      push(box[m][0], box[m][1], sqrt(box[m][0] * box[m][0] + box[m][1] * box[m][1]), eta_of(box[m][0], box[m][1]));
   if (n < 4) {
     for (int e = 0; e < 4; ++e) {
       const int i0 = qord(e), i1 = qord((e + 1) & 3);
       const double y1 = q[i0][0], z1 = q[i0][1], y2 = q[i1][0], z2 = q[i1][1];
       double h[2][2];
-      int nh = seg_circle(y1, z1, y2, z2, rmin, h);
-      for (int k = 0; k < nh; ++k) {
-        const double E = adj_eta(eta_of(h[k][0], h[k][1]), emin, emax);
-        if (E >= emin - kGeomEps && E <= emax + kGeomEps && n < kMaxVerts) {
-          ed[n][0] = h[k][0]; ed[n][1] = h[k][1]; ++n;
-        }
-      }
-      nh = seg_circle(y1, z1, y2, z2, rmax, h);
-      for (int k = 0; k < nh; ++k) {
-        const double E = adj_eta(eta_of(h[k][0], h[k][1]), emin, emax);
-        if (E >= emin - kGeomEps && E <= emax + kGeomEps && n < kMaxVerts) {
-          ed[n][0] = h[k][0]; ed[n][1] = h[k][1]; ++n;
+      for (int c = 0; c < 2; ++c) {
+        const int nh = seg_circle(y1, z1, y2, z2, c ? rmax : rmin, h);
+        for (int k = 0; k < nh; ++k) {
+          const double E0 = eta_of(h[k][0], h[k][1]), E = adj_eta(E0, emin, emax);
+          if (E >= emin - kGeomEps && E <= emax + kGeomEps)
+            push(h[k][0], h[k][1], sqrt(h[k][0] * h[k][0] + h[k][1] * h[k][1]), E0);
         }
       }
       double hy, hz;
-      if (seg_ray(y1, z1, y2, z2, emin, &hy, &hz)) {
-        const double R = sqrt(hy * hy + hz * hz);
-        if (R >= rmin - kGeomEps && R <= rmax + kGeomEps && n < kMaxVerts) { ed[n][0] = hy; ed[n][1] = hz; ++n; }
-      }
-      if (seg_ray(y1, z1, y2, z2, emax, &hy, &hz)) {
-        const double R = sqrt(hy * hy + hz * hz);
-        if (R >= rmin - kGeomEps && R <= rmax + kGeomEps && n < kMaxVerts) { ed[n][0] = hy; ed[n][1] = hz; ++n; }
-      }
+      for (int c = 0; c < 2; ++c)
+        if (seg_ray(y1, z1, y2, z2, c ? eb.shi : eb.slo, c ? eb.chi : eb.clo, &hy, &hz)) {
+          const double R = sqrt(hy * hy + hz * hz);
+          if (R >= rmin - kGeomEps && R <= rmax + kGeomEps) push(hy, hz, R, eta_of(hy, hz));
+        }
     }
   }
-  if (n < 3) return 0.0;
-  // unique vertices inside the bin (a vertex equal to a later one is dropped)
-  double uv[kMaxVerts][2];
+  if (nv < 3) return 0.0;
+  // unique vertices (a vertex equal to a later one is dropped)
   int nu = 0;
-  for (int i = 0; i < n; ++i) {
+  for (int i = 0; i < nv; ++i) {
     bool drop = false;
-    for (int j = i + 1; j < n; ++j) {
+    for (int j = i + 1; j < nv; ++j) {
       const double dy = ed[i][0] - ed[j][0], dz = ed[i][1] - ed[j][1];
-      if (sqrt(dy * dy + dz * dz) == 0) drop = true;
+      if (dy * dy + dz * dz == 0) drop = true;
     }
-    const double R = sqrt(ed[i][0] * ed[i][0] + ed[i][1] * ed[i][1]);
-    double E = eta_of(ed[i][0], ed[i][1]);
-    if (!within(E, emin, emax)) {
-      if (within(E + 360, emin, emax)) E += 360;
-      else if (within(E - 360, emin, emax)) E -= 360;
-    }
-    if (!within(R, rmin, rmax)) drop = true;
-    if (!within(E, emin, emax)) drop = true;
-    if (!drop) { uv[nu][0] = ed[i][0]; uv[nu][1] = ed[i][1]; ++nu; }
+    if (!drop) { ed[nu][0] = ed[i][0]; ed[nu][1] = ed[i][1]; ++nu; }
   }
   if (nu < 3) return 0.0;
-  return poly_area(uv, nu, rmin, rmax);
+  return poly_area(ed, nu, rmin, rmax);
 }
 
 struct Entry {
@@ -309,14 +315,17 @@ MI_HD inline void pixel_entries(const MapGeom &g, const MapBins &B, int i, int j
       const double scz = ((double)(2 * sj + 1) / (2.0 * spl)) - 0.5;
       const double dys[2] = {dyl, dyh}, dzs[2] = {dzl, dzh};
       double emi = 1800, ema = -1800, rmi = 1e8, rma = -1000;
-      double q[4][2];
+      double q[4][2], qR[4], qE[4];
       for (int k = 0; k < 2; ++k)
         for (int l = 0; l < 2; ++l) {
           double R, E;
           pix_to_reta(g, ypr + dys[k], zpr + dzs[l], &R, &E);
           emi = fmin(emi, E); ema = fmax(ema, E);
           rmi = fmin(rmi, R); rma = fmax(rma, R);
-          reta_to_yz(R, E, &q[k * 2 + l][0], &q[k * 2 + l][1]);
+          const int m = k * 2 + l;
+          reta_to_yz(R, E, &q[m][0], &q[m][1]);
+          qR[m] = sqrt(q[m][0] * q[m][0] + q[m][1] * q[m][1]);
+          qE[m] = eta_of(q[m][0], q[m][1]);
         }
       double Rt, Et;
       pix_to_reta(g, ypr + scy, zpr + scz, &Rt, &Et);
@@ -333,10 +342,47 @@ MI_HD inline void pixel_entries(const MapGeom &g, const MapBins &B, int i, int j
         ehi = 360 + elo;
         elo = t;
       }
+      // eta bins overlapping [elo, ehi], also a turn away, in ascending order: with ascending
+      // edges each turn's are one range
+      const double turn[3] = {0.0, 360.0, -360.0};
+      int k0[3], k1[3], kb = 0, ke_end = B.n_eta;
+      if (B.sorted) {
+        kb = B.n_eta;
+        ke_end = 0;
+        for (int t = 0; t < 3; ++t) {
+          const double a0 = elo + turn[t], b0 = ehi + turn[t];
+          int u = 0, v = B.n_eta;
+          while (u < v) {   // first bin with an upper edge >= a0
+            const int mid = (u + v) >> 1;
+            if (B.ehi[mid] >= a0) v = mid;
+            else u = mid + 1;
+          }
+          k0[t] = u;
+          v = B.n_eta;
+          while (u < v) {   // first bin with a lower edge > b0
+            const int mid = (u + v) >> 1;
+            if (B.elo[mid] <= b0) u = mid + 1;
+            else v = mid;
+          }
+          k1[t] = u;
+          if (k0[t] < k1[t]) {
+            kb = k0[t] < kb ? k0[t] : kb;
+            ke_end = k1[t] > ke_end ? k1[t] : ke_end;
+          }
+        }
+      }
       for (int kr = lo; kr < B.n_r && B.rlo[kr] <= rma; ++kr) {
         if (!(B.rhi[kr] >= rmi)) continue;
         const double rmin = B.rlo[kr], rmax = B.rhi[kr];
-        for (int ke = 0; ke < B.n_eta; ++ke) {
+        for (int ke = kb; ke < ke_end; ++ke) {
+          if (B.sorted) {
+            // on to the next bin of a range
+            int nx = ke_end;
+            for (int t = 0; t < 3; ++t)
+              if (k0[t] < k1[t] && ke < k1[t]) nx = (ke > k0[t] ? ke : k0[t]) < nx ? (ke > k0[t] ? ke : k0[t]) : nx;
+            ke = nx;
+            if (ke >= ke_end) break;
+          }
           const double a = B.elo[ke], b = B.ehi[ke];
           if (!((b >= elo && a <= ehi) || (b >= elo + 360 && a <= ehi + 360) ||
                 (b >= elo - 360 && a <= ehi - 360)))
@@ -346,7 +392,8 @@ MI_HD inline void pixel_entries(const MapGeom &g, const MapBins &B, int i, int j
             if (si == 0 && sj == 0) mask(bin);
             continue;
           }
-          const double A = quad_bin_area(q, rmin, rmax, a, b);
+          const EtaBin eb{a, b, B.slo[ke], B.clo[ke], B.shi[ke], B.chi[ke]};
+          const double A = quad_bin_area(q, qR, qE, rmin, rmax, eb);
           if (A < 1e-5) continue;
           double corr = A;
           if (g.sa || g.pol) {
@@ -376,32 +423,62 @@ MI_HD inline void pixel_entries(const MapGeom &g, const MapBins &B, int i, int j
 // ---------------------------------------------------------------------------
 // device build
 // ---------------------------------------------------------------------------
-__global__ void k_map_count(MapGeom g, MapBins B, const uint8_t *mask, int32_t *cnt, int32_t *bin_mask) {
+// sines and cosines of the eta edges: {lo, hi} of each bin, once per map instead of per overlap
+__global__ void k_map_trig(MapBins B, double *slo, double *clo, double *shi, double *chi) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= B.n_eta) return;
+  slo[t] = sin(B.elo[t] * kD2R);
+  clo[t] = cos(B.elo[t] * kD2R);
+  shi[t] = sin(B.ehi[t] * kD2R);
+  chi[t] = cos(B.ehi[t] * kD2R);
+}
+
+// Records of every `step`-th pixel, summed: the size of the whole map within a few per cent.
+__global__ void k_map_sample(MapGeom g, MapBins B, const uint8_t *mask, int step, unsigned long long *n_out) {
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * step;
+  if (t >= (int64_t)g.ny * g.nz) return;
+  const int i = (int)(t / g.nz), j = (int)(t % g.nz);
+  if (mask && mask[(int64_t)j * g.ny + i]) return;
+  unsigned long long n = 0;
+  pixel_entries(g, B, i, j, false, [&](int32_t, const mi_map_record &) { ++n; }, [&](int32_t) {});
+  atomicAdd(n_out, n);
+}
+
+// Every pixel's records, in the order in which threads reach them: where they go in pixel order
+// (seq: the record's number within its pixel) is known when all pixels have been counted.  One
+// evaluation of the geometry, which is all of the cost; records past `cap` are counted only.
+struct MapEntry {
+  int32_t bin, pix, seq, pad;
+  mi_map_record rec;
+};
+
+__global__ void __launch_bounds__(128) k_map_entries(MapGeom g, MapBins B, const uint8_t *mask, int32_t *cnt,
+                                                     int32_t *bin_mask, int32_t *bin_counts, MapEntry *ent,
+                                                     unsigned long long cap, unsigned long long *n_ent) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)g.ny * g.nz) return;
   const int i = (int)(t / g.nz), j = (int)(t % g.nz);
   const bool m = mask && mask[(int64_t)j * g.ny + i];
   int32_t n = 0;
-  pixel_entries(g, B, i, j, m, [&](int32_t, const mi_map_record &) { ++n; },
+  pixel_entries(g, B, i, j, m,
+                [&](int32_t bin, const mi_map_record &r) {
+                  const unsigned long long o = atomicAdd(n_ent, 1ull);
+                  if (o < cap) ent[o] = MapEntry{bin, (int32_t)t, n, 0, r};
+                  atomicAdd(bin_counts + bin, 1);
+                  ++n;
+                },
                 [&](int32_t bin) { bin_mask[bin] = 1; });
   cnt[t] = n;
 }
 
-__global__ void k_map_fill(MapGeom g, MapBins B, const uint8_t *mask, const int64_t *off, int32_t *keys,
-                           mi_map_record *recs, int32_t *bin_counts) {
+// the entries in pixel order
+__global__ void k_map_place(const MapEntry *ent, int64_t n, const int64_t *off, int32_t *keys, mi_map_record *recs) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)g.ny * g.nz) return;
-  const int i = (int)(t / g.nz), j = (int)(t % g.nz);
-  const bool m = mask && mask[(int64_t)j * g.ny + i];
-  int64_t o = off[t];
-  pixel_entries(g, B, i, j, m,
-                [&](int32_t bin, const mi_map_record &r) {
-                  keys[o] = bin;
-                  recs[o] = r;
-                  atomicAdd(bin_counts + bin, 1);
-                  ++o;
-                },
-                [&](int32_t) {});
+  if (t >= n) return;
+  const MapEntry e = ent[t];
+  const int64_t o = off[e.pix] + e.seq;
+  keys[o] = e.bin;
+  recs[o] = e.rec;
 }
 
 __global__ void k_gather_recs(const int32_t *idx, const mi_map_record *src, mi_map_record *dst, int64_t n) {
@@ -416,8 +493,14 @@ __global__ void k_iota(int32_t *v, int64_t n) {
 
 }  // namespace mi
 
+// The records are on the host (host build) or still on the device (device build: mi_map_copy
+// brings them straight into the caller's buffer).
 struct mi_map {
   std::vector<mi_map_record> recs;
+  mi_map_record *d_recs = nullptr;
+  int64_t n_recs = 0;
+  int device = -1;
+  cudaStream_t st = nullptr;
   std::vector<int32_t> nmap;      // pairs
   std::vector<int32_t> bin_mask;  // n_bins
   int64_t n_bins = 0;
@@ -453,6 +536,12 @@ static int make_geom(const mi_geometry *gi, const mi_binning *b, MapGeom *g) {
   return MI_OK;
 }
 
+static bool ascending(const double *v, int n) {
+  for (int k = 1; k < n; ++k)
+    if (!(v[k] >= v[k - 1])) return false;
+  return true;
+}
+
 static void finish_map(mi_map *m, int64_t n_bins, const std::vector<int32_t> &bin_counts) {
   m->n_bins = n_bins;
   m->nmap.resize(2 * n_bins);
@@ -464,7 +553,19 @@ static void finish_map(mi_map *m, int64_t n_bins, const std::vector<int32_t> &bi
   }
 }
 
-static int build_host(const MapGeom &g, const MapBins &B, const uint8_t *mask, mi_map *m) {
+static int build_host(const MapGeom &g, const MapBins &Bh, const uint8_t *mask, mi_map *m) {
+  MapBins B = Bh;
+  std::vector<double> trig(4 * (size_t)B.n_eta);
+  for (int k = 0; k < B.n_eta; ++k) {
+    trig[k] = sin(B.elo[k] * kD2R);
+    trig[B.n_eta + k] = cos(B.elo[k] * kD2R);
+    trig[2 * B.n_eta + k] = sin(B.ehi[k] * kD2R);
+    trig[3 * B.n_eta + k] = cos(B.ehi[k] * kD2R);
+  }
+  B.slo = trig.data();
+  B.clo = B.slo + B.n_eta;
+  B.shi = B.clo + B.n_eta;
+  B.chi = B.shi + B.n_eta;
   const int64_t n_bins = (int64_t)B.n_r * B.n_eta;
   m->bin_mask.assign(n_bins, 0);
   const int nthr = omp_get_max_threads();
@@ -491,11 +592,23 @@ static int build_host(const MapGeom &g, const MapBins &B, const uint8_t *mask, m
   if (total > INT32_MAX) return set_error(MI_E_RANGE, "mi_map_build: more than 2^31 map entries");
   finish_map(m, n_bins, counts);
   m->recs.resize(total);
+  m->n_recs = total;
   std::vector<int64_t> cur(n_bins);
   for (int64_t b = 0; b < n_bins; ++b) cur[b] = m->nmap[2 * b + 1];
   for (auto &v : cols)
     for (auto &e : v) m->recs[cur[e.bin]++] = e.rec;
   return MI_OK;
+}
+
+// host <-> device copies on the map's stream, in 4 MB pieces (pageable host memory)
+static cudaError_t map_copy_pieces(void *dst, const void *src, size_t bytes, cudaMemcpyKind kind, cudaStream_t st) {
+  constexpr size_t kPiece = size_t(4) << 20;
+  for (size_t o = 0; o < bytes; o += kPiece) {
+    cudaError_t e = cudaMemcpyAsync((uint8_t *)dst + o, (const uint8_t *)src + o, std::min(kPiece, bytes - o), kind, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // The whole build runs on a stream of its own with stream-ordered allocations: nothing in
@@ -505,29 +618,25 @@ static int build_device(const MapGeom &g, const MapBins &Bh, const uint8_t *mask
   const int64_t n_pix = (int64_t)g.ny * g.nz;
   const int64_t n_bins = (int64_t)Bh.n_r * Bh.n_eta;
   MI_CUDA(cudaSetDevice(device));
-  cudaStream_t st = nullptr;
-  MI_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  MI_CUDA(cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking));
+  m->device = device;
+  const cudaStream_t st = m->st;   // the map's own: its records are copied and freed on it
   std::vector<void *> owned;
   auto dalloc = [&](void **p, size_t bytes) -> cudaError_t {
     cudaError_t e = cudaMallocAsync(p, std::max<size_t>(bytes, 16), st);
     if (e == cudaSuccess) owned.push_back(*p);
     return e;
   };
+  auto dfree = [&](void *p) {
+    owned.erase(std::find(owned.begin(), owned.end(), p));
+    cudaFreeAsync(p, st);
+  };
   auto cleanup = [&]() {
     for (void *p : owned) cudaFreeAsync(p, st);
     cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
   };
-  // host <-> device copies on the build's stream, in 4 MB pieces (pageable host memory)
-  auto copy = [&](void *dst, const void *src, size_t bytes, cudaMemcpyKind kind) -> cudaError_t {
-    constexpr size_t kPiece = size_t(4) << 20;
-    for (size_t o = 0; o < bytes; o += kPiece) {
-      cudaError_t e = cudaMemcpyAsync((uint8_t *)dst + o, (const uint8_t *)src + o, std::min(kPiece, bytes - o),
-                                      kind, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+  auto copy = [&](void *dst, const void *src, size_t bytes, cudaMemcpyKind kind) {
+    return map_copy_pieces(dst, src, bytes, kind, st);
   };
 #define MI_DCHK(call)                                                     \
   do {                                                                    \
@@ -539,7 +648,7 @@ static int build_device(const MapGeom &g, const MapBins &Bh, const uint8_t *mask
     }                                                                     \
   } while (0)
   double *d_edges = nullptr;
-  MI_DCHK(dalloc((void **)&d_edges, sizeof(double) * (2 * Bh.n_r + 2 * Bh.n_eta)));
+  MI_DCHK(dalloc((void **)&d_edges, sizeof(double) * (2 * Bh.n_r + 6 * Bh.n_eta)));
   MI_DCHK(copy(d_edges, Bh.rlo, sizeof(double) * Bh.n_r, cudaMemcpyHostToDevice));
   MI_DCHK(copy(d_edges + Bh.n_r, Bh.rhi, sizeof(double) * Bh.n_r, cudaMemcpyHostToDevice));
   MI_DCHK(copy(d_edges + 2 * Bh.n_r, Bh.elo, sizeof(double) * Bh.n_eta, cudaMemcpyHostToDevice));
@@ -548,7 +657,15 @@ static int build_device(const MapGeom &g, const MapBins &Bh, const uint8_t *mask
   B.rlo = d_edges;
   B.rhi = d_edges + Bh.n_r;
   B.elo = d_edges + 2 * Bh.n_r;
-  B.ehi = d_edges + 2 * Bh.n_r + Bh.n_eta;
+  B.ehi = B.elo + Bh.n_eta;
+  double *trig = d_edges + 2 * Bh.n_r + 2 * Bh.n_eta;
+  k_map_trig<<<(unsigned)((Bh.n_eta + 127) / 128), 128, 0, st>>>(B, trig, trig + Bh.n_eta, trig + 2 * Bh.n_eta,
+                                                                 trig + 3 * Bh.n_eta);
+  MI_DCHK(cudaGetLastError());
+  B.slo = trig;
+  B.clo = trig + Bh.n_eta;
+  B.shi = trig + 2 * Bh.n_eta;
+  B.chi = trig + 3 * Bh.n_eta;
   uint8_t *d_mask = nullptr;
   if (mask_h) {
     MI_DCHK(dalloc((void **)&d_mask, n_pix));
@@ -556,16 +673,41 @@ static int build_device(const MapGeom &g, const MapBins &Bh, const uint8_t *mask
   }
   int32_t *d_cnt = nullptr, *d_bmask = nullptr, *d_bcnt = nullptr;
   int64_t *d_off = nullptr;
+  unsigned long long *d_n = nullptr;
   MI_DCHK(dalloc((void **)&d_cnt, sizeof(int32_t) * n_pix));
   MI_DCHK(dalloc((void **)&d_off, sizeof(int64_t) * (n_pix + 1)));
   MI_DCHK(dalloc((void **)&d_bmask, sizeof(int32_t) * n_bins));
   MI_DCHK(dalloc((void **)&d_bcnt, sizeof(int32_t) * n_bins));
+  MI_DCHK(dalloc((void **)&d_n, sizeof(unsigned long long)));
   MI_DCHK(cudaMemsetAsync(d_bmask, 0, sizeof(int32_t) * n_bins, st));
-  MI_DCHK(cudaMemsetAsync(d_bcnt, 0, sizeof(int32_t) * n_bins, st));
   const int thr = 128;
   const unsigned grid = (unsigned)((n_pix + thr - 1) / thr);
-  k_map_count<<<grid, thr, 0, st>>>(g, B, d_mask, d_cnt, d_bmask);
+  // room for the entries: a sample's estimate and a tenth more; where that falls short, the
+  // count is known and the second run has room for all
+  constexpr int kStep = 67;
+  unsigned long long total_u = 0;
+  MI_DCHK(cudaMemsetAsync(d_n, 0, sizeof(unsigned long long), st));
+  k_map_sample<<<(unsigned)((n_pix / kStep + thr) / thr), thr, 0, st>>>(g, B, d_mask, kStep, d_n);
   MI_DCHK(cudaGetLastError());
+  MI_DCHK(copy(&total_u, d_n, sizeof(total_u), cudaMemcpyDeviceToHost));
+  MapEntry *d_ent = nullptr;
+  unsigned long long cap = total_u * kStep + total_u * kStep / 10 + 65536;
+  for (int run = 0; run < 2; ++run) {
+    MI_DCHK(dalloc((void **)&d_ent, sizeof(MapEntry) * cap));
+    MI_DCHK(cudaMemsetAsync(d_bcnt, 0, sizeof(int32_t) * n_bins, st));
+    MI_DCHK(cudaMemsetAsync(d_n, 0, sizeof(unsigned long long), st));
+    k_map_entries<<<grid, thr, 0, st>>>(g, B, d_mask, d_cnt, d_bmask, d_bcnt, d_ent, cap, d_n);
+    MI_DCHK(cudaGetLastError());
+    MI_DCHK(copy(&total_u, d_n, sizeof(total_u), cudaMemcpyDeviceToHost));
+    if (total_u <= cap || total_u > INT32_MAX) break;
+    dfree(d_ent);
+    cap = total_u;
+  }
+  if (total_u > INT32_MAX) {
+    cleanup();
+    return set_error(MI_E_RANGE, "mi_map_build: more than 2^31 map entries");
+  }
+  const int64_t total = (int64_t)total_u;
   // exclusive scan of counts (int64)
   {
     size_t tmp_bytes = 0;
@@ -574,25 +716,20 @@ static int build_device(const MapGeom &g, const MapBins &Bh, const uint8_t *mask
     MI_DCHK(dalloc(&tmp, tmp_bytes));
     MI_DCHK(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, d_cnt, d_off, n_pix, st));
   }
-  int64_t last_off = 0;
-  int32_t last_cnt = 0;
-  MI_DCHK(copy(&last_off, d_off + n_pix - 1, sizeof(int64_t), cudaMemcpyDeviceToHost));
-  MI_DCHK(copy(&last_cnt, d_cnt + n_pix - 1, sizeof(int32_t), cudaMemcpyDeviceToHost));
-  const int64_t total = last_off + last_cnt;
-  if (total > INT32_MAX) {
-    cleanup();
-    return set_error(MI_E_RANGE, "mi_map_build: more than 2^31 map entries");
-  }
   int32_t *d_keys = nullptr, *d_keys2 = nullptr, *d_idx = nullptr, *d_idx2 = nullptr;
-  mi_map_record *d_recs = nullptr, *d_recs2 = nullptr;
+  mi_map_record *d_recs = nullptr;
   MI_DCHK(dalloc((void **)&d_keys, sizeof(int32_t) * total));
+  MI_DCHK(dalloc((void **)&d_recs, sizeof(mi_map_record) * total));
+  if (total > 0) {
+    k_map_place<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d_ent, total, d_off, d_keys, d_recs);
+    MI_DCHK(cudaGetLastError());
+  }
+  dfree(d_ent);   // before the sort's buffers: the build needs no more memory than its records twice
   MI_DCHK(dalloc((void **)&d_keys2, sizeof(int32_t) * total));
   MI_DCHK(dalloc((void **)&d_idx, sizeof(int32_t) * total));
   MI_DCHK(dalloc((void **)&d_idx2, sizeof(int32_t) * total));
-  MI_DCHK(dalloc((void **)&d_recs, sizeof(mi_map_record) * total));
-  MI_DCHK(dalloc((void **)&d_recs2, sizeof(mi_map_record) * total));
-  k_map_fill<<<grid, thr, 0, st>>>(g, B, d_mask, d_off, d_keys, d_recs, d_bcnt);
-  MI_DCHK(cudaGetLastError());
+  MI_DCHK(cudaMallocAsync((void **)&m->d_recs, std::max<size_t>(sizeof(mi_map_record) * total, 16), st));
+  mi_map_record *d_recs2 = m->d_recs;
   if (total > 0) {
     k_iota<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d_idx, total);
     MI_DCHK(cudaGetLastError());
@@ -610,13 +747,13 @@ static int build_device(const MapGeom &g, const MapBins &Bh, const uint8_t *mask
   }
   std::vector<int32_t> counts(n_bins);
   m->bin_mask.resize(n_bins);
-  m->recs.resize(total);
+  m->n_recs = total;
   MI_DCHK(copy(counts.data(), d_bcnt, sizeof(int32_t) * n_bins, cudaMemcpyDeviceToHost));
   MI_DCHK(copy(m->bin_mask.data(), d_bmask, sizeof(int32_t) * n_bins, cudaMemcpyDeviceToHost));
-  if (total > 0)
-    MI_DCHK(copy(m->recs.data(), d_recs2, sizeof(mi_map_record) * total, cudaMemcpyDeviceToHost));
   finish_map(m, n_bins, counts);
-  cleanup();
+  for (void *p : owned) cudaFreeAsync(p, st);
+  owned.clear();
+  MI_DCHK(cudaStreamSynchronize(st));
 #undef MI_DCHK
   return MI_OK;
 }
@@ -630,6 +767,7 @@ int mi_map_build(const mi_geometry *geom, const mi_binning *bins, int device, mi
   int rc = make_geom(geom, bins, &g);
   if (rc) return rc;
   MapBins B{bins->n_r, bins->n_eta, bins->r_lo, bins->r_hi, bins->eta_lo, bins->eta_hi};
+  B.sorted = ascending(bins->eta_lo, bins->n_eta) && ascending(bins->eta_hi, bins->n_eta);
   mi_map *m = new (std::nothrow) mi_map();
   if (!m) return set_error(MI_E_OOM, "mi_map_build: host allocation failed");
   if (device < 0) {
@@ -646,7 +784,7 @@ int mi_map_build(const mi_geometry *geom, const mi_binning *bins, int device, mi
     cudaSetDevice(prev);
   }
   if (rc) {
-    delete m;
+    mi_map_destroy(m);
     return rc;
   }
   *out = m;
@@ -655,7 +793,7 @@ int mi_map_build(const mi_geometry *geom, const mi_binning *bins, int device, mi
 
 int mi_map_sizes(const mi_map *m, int64_t *n_records, int64_t *n_bins) {
   if (!m) return set_error(MI_E_ARG, "mi_map_sizes: null map");
-  if (n_records) *n_records = (int64_t)m->recs.size();
+  if (n_records) *n_records = m->n_recs;
   if (n_bins) *n_bins = m->n_bins;
   return MI_OK;
 }
@@ -663,11 +801,32 @@ int mi_map_sizes(const mi_map *m, int64_t *n_records, int64_t *n_bins) {
 int mi_map_copy(const mi_map *m, mi_map_record *records, int32_t *nmap, int32_t *bin_mask) {
   if (!m) return set_error(MI_E_ARG, "mi_map_copy: null map");
   if (records && !m->recs.empty()) memcpy(records, m->recs.data(), m->recs.size() * sizeof(mi_map_record));
+  if (records && m->d_recs && m->n_recs > 0) {
+    int prev = 0;
+    cudaGetDevice(&prev);
+    MI_CUDA(cudaSetDevice(m->device));
+    const cudaError_t e =
+        map_copy_pieces(records, m->d_recs, m->n_recs * sizeof(mi_map_record), cudaMemcpyDeviceToHost, m->st);
+    cudaSetDevice(prev);
+    MI_CUDA(e);
+  }
   if (nmap) memcpy(nmap, m->nmap.data(), m->nmap.size() * sizeof(int32_t));
   if (bin_mask) memcpy(bin_mask, m->bin_mask.data(), m->bin_mask.size() * sizeof(int32_t));
   return MI_OK;
 }
 
-void mi_map_destroy(mi_map *m) { delete m; }
+void mi_map_destroy(mi_map *m) {
+  if (!m) return;
+  if (m->st) {
+    int prev = 0;
+    cudaGetDevice(&prev);
+    cudaSetDevice(m->device);
+    if (m->d_recs) cudaFreeAsync(m->d_recs, m->st);
+    cudaStreamSynchronize(m->st);
+    cudaStreamDestroy(m->st);
+    cudaSetDevice(prev);
+  }
+  delete m;
+}
 
 }  // extern "C"

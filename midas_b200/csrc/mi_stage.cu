@@ -28,13 +28,41 @@ namespace mi {
 // 16-byte granule of frames 16g .. 16g+15 at position g ^ (c % 8): the 128-byte swizzle
 // phase the tensor-core operand of a K slot with k % 8 == c % 8 expects, so a run of
 // consecutive pixels is staged with one plain bulk copy per plane.
-constexpr int kXcLoads = 8;
+// How a chunk's 8-pixel groups are read: one element at a time (8-bit frames), as 16-byte pieces
+// (16-bit frames whose rows all start on 16 bytes), or as two such pieces around the group, put
+// together by its offset in them (any other 16-bit frames: an odd width or stride).  Element
+// loads of 16-bit frames touch each sector eight times: 100 frames of 1475 x 1679 took 363 us,
+// with the pieces 235 (1.13 GB: 4.8 TB/s).
+enum { kXcElem, kXcVec, kXcShift };
+// groups in flight per thread: of two pieces each, eight take the registers of a block more per SM
+// (334 us with 8, 235 with 4 or 2; aligned groups 260 us with 8, 344 with 4 on the 2880^2 sweep)
+__host__ __device__ constexpr int xc_loads(int load) { return load == kXcShift ? 4 : 8; }
 
-template <typename T, bool VEC, bool PLANES>
+// Eight 16-bit pixels from any even address: the 16-byte pieces that hold them.  Both pieces hold
+// at least one of the pixels, so neither lies outside the frames' pages.
+__device__ __forceinline__ uint4 xc_shifted(const uint16_t *src) {
+  const uint32_t mis = (uint32_t)((uintptr_t)src & 15u);
+  const uint4 *p = (const uint4 *)((uintptr_t)src - mis);
+  const uint4 a = __ldg(p);
+  if (mis == 0) return a;
+  const uint4 b = __ldg(p + 1);
+  const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  uint32_t t[6], u[5];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) t[k] = (mis & 8u) ? w[k + 2] : w[k];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) u[k] = (mis & 4u) ? t[k + 1] : t[k];
+  const uint32_t sh = (mis & 2u) * 8u;
+  return make_uint4(__funnelshift_r(u[0], u[1], sh), __funnelshift_r(u[1], u[2], sh),
+                    __funnelshift_r(u[2], u[3], sh), __funnelshift_r(u[3], u[4], sh));
+}
+
+template <typename T, int LOAD, bool PLANES>
 __global__ void __launch_bounds__(256) k_xc(const T *__restrict__ frames, int64_t stride, int F, int ny, int z_off,
                                             const XcChunk *__restrict__ chunks, uint8_t *__restrict__ xc,
                                             int64_t n_xc) {
   constexpr int kPitch = kXcRowBytes / 2;  // u16 per compact pixel
+  constexpr int kXcLoads = xc_loads(LOAD);
   __shared__ __align__(16) uint16_t S[kXcFrames][kXcChunk + 8];
   const XcChunk ch = chunks[blockIdx.x];
   const int nv = (ch.n + 7) >> 3;  // groups of 8 pixels
@@ -55,8 +83,10 @@ __global__ void __launch_bounds__(256) k_xc(const T *__restrict__ frames, int64_
         val[u] = make_uint4(0u, 0u, 0u, 0u);
         if (i < n_items && f < fh) {
           const T *src = frames + (int64_t)(h * kXcFrames + f) * stride + base + 8 * v;
-          if constexpr (VEC) {
+          if (LOAD == kXcVec) {
             val[u] = __ldg((const uint4 *)src);
+          } else if (LOAD == kXcShift && 8 * v + 8 <= ch.n) {
+            val[u] = xc_shifted((const uint16_t *)src);
           } else {
             uint32_t t[4];
 #pragma unroll
@@ -169,19 +199,19 @@ int launch_xc(Plan *p, int panel, const void *frames, int dtype, int F, int64_t 
       const bool vec = ((uintptr_t)frames % 16 == 0) && ((stride * 2) % 16 == 0) && ((pn.ny * 2) % 16 == 0);
       const uint16_t *f16 = (const uint16_t *)frames;
       if (vec && planes)
-        k_xc<uint16_t, true, true><<<grid, 256, 0, s>>>(f16, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
+        k_xc<uint16_t, kXcVec, true><<<grid, 256, 0, s>>>(f16, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
       else if (vec)
-        k_xc<uint16_t, true, false><<<grid, 256, 0, s>>>(f16, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
+        k_xc<uint16_t, kXcVec, false><<<grid, 256, 0, s>>>(f16, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
       else if (planes)
-        k_xc<uint16_t, false, true><<<grid, 256, 0, s>>>(f16, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
+        k_xc<uint16_t, kXcShift, true><<<grid, 256, 0, s>>>(f16, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
       else
-        k_xc<uint16_t, false, false><<<grid, 256, 0, s>>>(f16, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
+        k_xc<uint16_t, kXcShift, false><<<grid, 256, 0, s>>>(f16, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
     } else if (dtype == MI_DT_U8) {
       const uint8_t *f8 = (const uint8_t *)frames;
       if (planes)
-        k_xc<uint8_t, false, true><<<grid, 256, 0, s>>>(f8, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
+        k_xc<uint8_t, kXcElem, true><<<grid, 256, 0, s>>>(f8, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
       else
-        k_xc<uint8_t, false, false><<<grid, 256, 0, s>>>(f8, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
+        k_xc<uint8_t, kXcElem, false><<<grid, 256, 0, s>>>(f8, stride, F, pn.ny, pn.z_off, chunks, p->d_xc, p->n_xc);
     } else {
       return set_error(MI_E_ARG, "launch_xc: dtype %d does not fit u16 staging", dtype);
     }

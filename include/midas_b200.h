@@ -242,9 +242,10 @@ void mi_plan_destroy(mi_plan *plan);
 
 /* Host -> device copy of F frames for this plan: only the pixels the map can read cross
  * PCIe.  Per group of 16 detector rows of the referenced band (ref_row_lo .. ref_row_hi-1)
- * the columns any row of the group references (rounded out to 8 pixels), all F frames in one
- * 3-D copy on `stream` (upload_pixels of mi_plan_info per frame); when a stride is not a
- * whole number of rows, the band's full rows in one 2-D copy.  The other pixels of the
+ * the columns any row of the group references (rounded out to 8 pixels; upload_pixels of
+ * mi_plan_info per frame).  Page-locked frames of up to 1 MB per group go by one kernel that
+ * reads them over PCIe, others by one 3-D copy per group; when a stride is not a whole number
+ * of rows, the band's full rows in one 2-D copy.  All on `stream`.  The other pixels of the
  * device frames are left as they are, and no kernel reads them.  The reference copies every
  * whole frame (IntegratorFitPeaksGPUStream.cu:1633-1683).  `host` should be page-locked for
  * the copy to be asynchronous. */
@@ -289,8 +290,8 @@ int mi_integrate_batch_static(mi_plan *plan, const void *frames, int dtype, int 
                               double *lineout_sm, void *stream);
 
 /* The reference's own GPU algorithm, one frame per launch: cast/dark kernel, one thread per
- * bin in heaviest-first order with FP32 accumulation and on-the-fly bilinear sampling in
- * gradient mode, FP64 cake, then the two profile kernels.  This is the plain baseline. */
+ * bin with FP32 accumulation in record order and bilinear sampling at the FP32 positions (worked
+ * out once, with the plan) in gradient mode, FP64 cake, then the two profile kernels. */
 int mi_integrate_plain(mi_plan *plan, const void *frame, int dtype, double *cake,
                        double *lineout_aw, double *lineout_sm, void *stream);
 

@@ -497,7 +497,8 @@ int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t st
 // 996 / 765, 1131 / 1241, 1675 / 2201.  CSR kernel / this, 16 frames: 139 / 91, 703 / 291, 1036 / 413,
 // 1807 / 784.  MMA kernel / this: 8 frames 147 / 66, 149 / 80, 513 / 226, 581 / 312, 804 / 452 (1024^2
 // floor and bilinear, 2048^2 floor and gradient, 2880^2); 16 frames 148 / 124, 151 / 155, 519 / 451,
-// 589 / 616, 816 / 898.
+// 589 / 616, 816 / 898.  (Run and MMA plans whose pixel-major buffer holds a block of eight frames leave
+// this path earlier, below.)
 constexpr int kOneFrames = 16, kOneFramesMma = 12;
 constexpr int kOneChunk = 8;     // frames whose bin results are held for the lineouts
 // Run plans from kOnePmMin frames on: eight frames of a pixel side by side (launch_one_pm), for 8/16-bit
@@ -507,6 +508,11 @@ constexpr int kOneChunk = 8;     // frames whose bin results are held for the li
 // 3960 x 360 gradient); u16, 32 frames 1007 / 488, 1136 / 786, 628 / 572; 48 frames 1024 / 762, 1163 /
 // 1189, 652 / 855.
 constexpr int kOnePmMin = 5, kOnePmU16 = 32;
+// MMA plans from kOnePmMinMma to kOnePmMma frames.  MMA kernel / this, us: 4 frames 146 / 48, 510 / 96, 578
+// / 116, 799 / 228 (1024^2, 2048^2 floor and gradient, 2880^2); 24 frames 150 / 77, 526 / 207, 599 / 326,
+// 829 / 670; 32 frames 151 / 88, 530 / 255, 609 / 425, 839 / 909.  Over frames / this: 2 frames 37, 64, 84,
+// 138 against one block of eight; 4 frames 49 / 48, 128 / 96, 186 / 116, 237 / 228.
+constexpr int kOnePmMinMma = 3, kOnePmMma = 24;
 int build_one(Plan *p, size_t *acct);
 bool one_pm_fits(const Plan *p, bool want_lo);
 // frames [first, first + F) of every panel; cake and partial are those of the first

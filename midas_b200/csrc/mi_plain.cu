@@ -296,12 +296,18 @@ int build_plain(Plan *p, const mi_map_record *recs, const int32_t *nmap, size_t 
     int32_t *d_nmap = nullptr;
     int64_t *d_n = nullptr;
     mi_map_record *d_recs = nullptr;
-    MI_CUDA(temp((void **)&d_nmap, sizeof(int32_t) * 2 * p->n_bins));
-    MI_CUDA(copy_pieces(d_nmap, nmap, sizeof(int32_t) * 2 * p->n_bins, cudaMemcpyHostToDevice));
-    MI_CUDA(temp((void **)&d_n, sizeof(int64_t) * g.n_slices));
-    MI_CUDA(temp((void **)&d_recs, sizeof(mi_map_record) * p->n_records));
-    if (p->n_records > 0)
-      MI_CUDA(copy_pieces(d_recs, recs, sizeof(mi_map_record) * p->n_records, cudaMemcpyHostToDevice));
+    // the map on the device while its layout is made: in the pixel-major buffer, which is large
+    // enough for most maps and not in use yet, else in scratch
+    const size_t b_recs = sizeof(mi_map_record) * p->n_records, b_n = sizeof(int64_t) * g.n_slices;
+    const size_t b_nmap = sizeof(int32_t) * 2 * p->n_bins, need = b_recs + b_n + b_nmap;
+    uint8_t *at = p->d_xc;
+    if (!at || (size_t)p->n_xc * kXcRowBytes < need) MI_CUDA(temp((void **)&at, need));
+    d_recs = (mi_map_record *)at;
+    d_n = (int64_t *)(at + b_recs);
+    d_nmap = (int32_t *)(at + b_recs + b_n);
+    MI_CUDA(copy_pieces(d_nmap, nmap, b_nmap, cudaMemcpyHostToDevice));
+    if (p->n_records > 0) MI_CUDA(copy_pieces(d_recs, recs, b_recs, cudaMemcpyHostToDevice));
+    MI_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // a pageable copy's last piece may still be under way
     MI_CUDA(keep((void **)&p->d_plain_cnt, sizeof(int32_t) * 32 * g.n_slices));
     MI_CUDA(keep((void **)&p->d_plain_ptr, sizeof(int64_t) * g.n_slices));
     MI_CUDA(keep((void **)&p->d_area_gs, sizeof(float) * p->n_bins));

@@ -241,8 +241,9 @@ class CakePlan:
         """Copy host frames (CPU tensor (F, NZ, NY), page-locked for an asynchronous copy) to
         device frames of the same shape and dtype: only the pixels the map can read cross
         PCIe -- per group of 16 rows of the referenced band, the columns the group references
-        (``info["upload_pixels"]`` per frame), one 3-D copy per group; the device frames'
-        other pixels are left as they are."""
+        (``info["upload_pixels"]`` per frame), by one kernel (page-locked frames, up to 1 MB
+        per group) or one 3-D copy per group; the device frames' other pixels are left as
+        they are."""
         if host_frames.device.type != "cpu" or device_frames.device != self.device:
             raise ValueError("upload copies a CPU tensor into a tensor on the plan's device")
         if host_frames.dtype != device_frames.dtype or host_frames.shape[0] > device_frames.shape[0]:

@@ -185,8 +185,8 @@ class DeviceBackend:
     arm of the serving benchmark.
 
     ``small_batch``: batches of at most this many frames go through that one-frame kernel
-    too (the batched kernels' cost per launch hardly depends on the frame count, and for
-    one frame the one-frame kernel is 1.5 to 4 times faster); larger batches use the
+    too (on the reference algorithm's sums and FP64 cake; a batched call of one frame takes
+    about as long); larger batches use the
     stream's batched encoding.  A frame's result then depends on which path served it,
     never on the other frames of its batch.
 

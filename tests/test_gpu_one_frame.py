@@ -58,9 +58,9 @@ def test_few_frames_equal_the_batch(cuda, enc, rows, mode, sem, var, n_r, n_eta)
 @pytest.mark.parametrize("mode,sem,var", [("floor", "py", False), ("gradient", "py", True), ("bilinear", "ic", False)])
 @pytest.mark.parametrize("n_r,n_eta", [(1, 1), (13, 2), (50, 7), (24, 40)])
 def test_few_frames_equal_the_batch_on_the_tensor_cores(cuda, mode, sem, var, n_r, n_eta):
-    """MMA plans: 1 to 12 frames by the lane-per-bin kernel, 20 by the tensor cores; the first
-    call after a dark is set or cleared follows it."""
-    ny, nz, F = 61, 53, 20
+    """MMA plans: few frames by the lane-per-bin kernels, 70 by the tensor cores; the first call
+    after a dark is set or cleared follows it."""
+    ny, nz, F = 61, 53, 70
     rng = np.random.default_rng(n_eta)
     plan = CakePlan(_map(n_r, n_eta, ny, nz, n_r), n_r=n_r, n_eta=n_eta, n_pixels_y=ny, n_pixels_z=nz, mode=mode,
                     semantics=sem, variance=var, bc_y=30.1, bc_z=26.4, device=cuda, encoding="mma")
@@ -68,7 +68,7 @@ def test_few_frames_equal_the_batch_on_the_tensor_cores(cuda, mode, sem, var, n_
         plan.set_dark(dark)
         for dt, top in ((np.uint8, 256), (np.uint16, 65536)):
             frames = torch.from_numpy(rng.integers(0, top, (F, nz, ny)).astype(dt)).to(cuda)
-            parts = [(f, n, plan.integrate(frames[f:f + n])) for f, n in ((0, 1), (3, 2), (4, 12), (10, 9))]
+            parts = [(f, n, plan.integrate(frames[f:f + n])) for f, n in ((0, 1), (3, 2), (7, 3), (4, 8), (10, 17), (2, 24), (5, 25))]
             whole = plan.integrate(frames)
             for f, n, part in parts:
                 for x, y in zip(part, whole):

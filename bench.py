@@ -778,7 +778,7 @@ def panel_bench(args, dev, reps=3):
            "ms_per_batch": round(ms, 3), "frame_sets_per_s": round(F / (ms / 1e3), 1),
            "panel_frames_per_s": round(len(ws) * F / (ms / 1e3), 1),
            "alg_gb_s": round((csr_map_bytes(info) + F * frame_bytes) / (ms / 1e3) / 1e9, 1),
-           "staging": "fp32 pixel-major (the int32 panel); one run-kernel launch per 64 frames for all panels",
+           "staging": "fp32, eight frames of a pixel side by side (the int32 panel); lane per bin",
            "setup_s": {"maps_gpu": round(t_map, 2), "plan_build": round(t_plan, 2)}}
     sample = (ws, maps, [f[0].cpu().numpy() for f in frames], darks, ck[0].cpu().numpy().reshape(-1),
               aw[0].cpu().numpy())

@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kClearSeries) k_fit_clear(const FitPlanArgs a)
 // model, the order of every sum and the iteration are fit_one_job's, bit for bit.
 // Bounded by FP64 issue and the solve's chain, not by memory.  fit_one_job (one column per warp,
 // the solve on lane 0 through shared memory) took 9.95 ms for 115,200 windows of 25 samples;
-// this takes 1.46 ms, same bits (9,000 windows: 2.56 -> 0.38 ms).
+// this takes 1.46 ms, same bits (1,800 windows of 19 samples: 2.56 -> 0.38 ms).
 constexpr int kEtaNP = 5, kEtaTri = kEtaNP * (kEtaNP + 1) / 2, kEtaNrm = kEtaTri + kEtaNP;
 
 __host__ __device__ inline uint32_t eta_slot_bytes(int n_max) {

@@ -1,7 +1,7 @@
 """Batched pseudo-Voigt peak fits on the device (kernel (d) of libmidas_b200).
 
 ``fit_batch`` fits every (frame, peak) window of a batch of lineouts in one launch,
-one warp per window; ``fit_peaks`` mirrors the single-lineout API of
+up to eight windows per warp; ``fit_peaks`` mirrors the single-lineout API of
 packages/midas_integrate/midas_integrate/peakfit.py:334 (output rows in the
 PF_PARAMS_PER_PEAK = 7 layout of FF_HEDM/src/PeakFit.h).
 

@@ -4,9 +4,8 @@
 // per pass over the map.  Here a lane is a bin.  A bin's terms {pixel, weight} are the ones of
 // the plan's tiles in the order in which the batched kernel adds them, with the ends of its
 // unit partials marked, so every FP64 sum, every rounding of a partial to FP32 and the scaling
-// are the batched kernel's: a frame's cake and lineouts are the same bits on either path.  (A
-// pixel that is not finite reaches the bins whose terms hold it; the run kernel's zero weights
-// spread it to other bins of the same strip.)
+// are the batched kernel's: a frame's cake and lineouts are the same bits on either path, and a
+// pixel or dark that is not finite reaches the bins whose terms hold it on both.
 //
 // MMA plans: the terms carry the fixed-point weights, the sums are exact 64-bit integers and are
 // scaled as the tensor-core kernel's epilogue scales them: the same bits again.

@@ -532,6 +532,10 @@ int launch_xc(Plan *p, int panel, const void *frames, int dtype, int F, int64_t 
 // Upload of page-locked host frames by one kernel; false when it does not apply
 bool launch_upload(const Plan *p, const void *host, int es, int n_frames, int64_t host_stride, void *dev,
                    int64_t dev_stride, cudaStream_t s);
+// whether it applies: the frames' device address, else null; and its test of a range of host memory
+const uint8_t *upload_source(const Plan *p, const void *host, int es, int n_frames, int64_t host_stride,
+                             const void *dev, int64_t dev_stride);
+bool range_holds(uint64_t start, uint64_t bytes, uint64_t first, uint64_t last);
 // Caking of frames [0, F) (F <= 128 u16 / 64 fp32) already staged pixel-major.
 int launch_runs_staged(Plan *p, bool as_f32, int F, float *cake, double *partial, bool want_lo, cudaStream_t s);
 // MMA encoding (mi_mma.cu): caking of frames [0, F) (F <= 128) staged as byte planes, and

@@ -1924,6 +1924,16 @@ int mi_upload_frames(const mi_plan *p, const void *host, int dtype, int n_frames
   return MI_OK;
 }
 
+// For the tests (not part of the C ABI): whether mi_upload_frames would read these host frames by
+// its kernel, and the test of their range on made-up addresses.  Neither touches the memory.
+int mi_test_upload_by_kernel(const mi_plan *p, const void *host, int dtype, int n_frames, int64_t host_stride,
+                             const void *device_frames, int64_t device_stride) {
+  return upload_source(p, host, (int)dtype_size(dtype), n_frames, host_stride, device_frames, device_stride) != nullptr;
+}
+int mi_test_range_holds(uint64_t start, uint64_t bytes, uint64_t first, uint64_t last) {
+  return range_holds(start, bytes, first, last);
+}
+
 int mi_integrate_plain(mi_plan *p, const void *frame, int dtype, double *cake, double *lo_aw,
                        double *lo_sm, void *stream) {
   if (!p || !frame) return set_error(MI_E_ARG, "mi_integrate_plain: null argument");

@@ -17,6 +17,7 @@
 // where alignment allows (u16), into shared memory with 16-byte groups XOR-swizzled by
 // frame octet so the transposed reads are conflict-free; then 16-byte stores, eight
 // consecutive threads writing one pixel's 128-byte row of a frame group.
+#include <cuda.h>
 #include <stdint.h>
 
 #include "mi_internal.h"
@@ -268,34 +269,68 @@ __global__ void __launch_bounds__(256) k_upload(const uint8_t *__restrict__ src,
   }
 }
 
-// true when the frames went by the kernel; false: the caller copies (pageable memory, row
-// addresses that differ modulo 16, or enough bytes per copy)
+// The page-locked range that a host address lies in, from the driver (no link to libcuda)
+static bool locked_range(const void *ptr, uint64_t *start, uint64_t *bytes) {
+  using Fn = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+  static const Fn query = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+                   q == cudaDriverEntryPointSuccess
+               ? (Fn)f
+               : nullptr;
+  }();
+  CUdeviceptr at = 0;
+  size_t n = 0;
+  if (!query || query(&at, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)(uintptr_t)ptr) != CUDA_SUCCESS ||
+      query(&n, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)(uintptr_t)ptr) != CUDA_SUCCESS)
+    return false;
+  *start = (uint64_t)at;
+  *bytes = (uint64_t)n;
+  return true;
+}
+
+bool range_holds(uint64_t start, uint64_t bytes, uint64_t first, uint64_t last) {
+  return start <= first && first <= last && last - start < bytes;
+}
+
+// the device's address of the frames when the kernel can read them, else null: the caller copies
+// (pageable memory, row addresses that differ modulo 16, or enough bytes per copy)
+const uint8_t *upload_source(const Plan *p, const void *host, int es, int n_frames, int64_t host_stride,
+                             const void *dev, int64_t dev_stride) {
+  const int64_t n = (int64_t)p->upload_groups.size();
+  if (!p->d_upload || n_frames > 65535 || p->upload_pixels * es * n_frames > n * kUploadKernelBytes) return nullptr;
+  // every row is read as 16-byte pieces at one alignment on both sides
+  if (((uintptr_t)host - (uintptr_t)dev) % 16 != 0) return nullptr;
+  if (n_frames > 1 && ((host_stride - dev_stride) * es) % 16 != 0) return nullptr;
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+  if ((uintptr_t)a.devicePointer % 16 != (uintptr_t)host % 16) return nullptr;
+  // one page-locked range holds the frames from the first byte to the last: buffers locked piece by
+  // piece may have pageable memory between the pieces, and their device addresses do not tell
+  const uint64_t first = (uint64_t)(uintptr_t)host;
+  const uint64_t last = first + (uint64_t)(((int64_t)(n_frames - 1) * host_stride + (int64_t)p->ny * p->nz) * es) - 1;
+  uint64_t start = 0, bytes = 0;
+  if (!locked_range(host, &start, &bytes) || !range_holds(start, bytes, first, last)) return nullptr;
+  return (const uint8_t *)a.devicePointer;
+}
+
 bool launch_upload(const Plan *p, const void *host, int es, int n_frames, int64_t host_stride, void *dev,
                    int64_t dev_stride, cudaStream_t s) {
-  const int64_t n = (int64_t)p->upload_groups.size();
-  if (!p->d_upload || n_frames > 65535 || p->upload_pixels * es * n_frames > n * kUploadKernelBytes) return false;
-  // every row is read as 16-byte pieces at one alignment on both sides
-  if (((uintptr_t)host - (uintptr_t)dev) % 16 != 0) return false;
-  if (n_frames > 1 && ((host_stride - dev_stride) * es) % 16 != 0) return false;
-  const uint8_t *first = (const uint8_t *)host;
-  const uint8_t *last = first + ((int64_t)(n_frames - 1) * host_stride + (int64_t)p->ny * p->nz) * es - 1;
-  cudaPointerAttributes a{}, b{};
-  if (cudaPointerGetAttributes(&a, first) != cudaSuccess || cudaPointerGetAttributes(&b, last) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  // page-locked from the first byte to the last, mapped at one offset
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer ||
-      (const uint8_t *)b.devicePointer - (const uint8_t *)a.devicePointer != last - first)
-    return false;
-  if ((uintptr_t)a.devicePointer % 16 != (uintptr_t)host % 16) return false;
   int prev = 0;
   cudaGetDevice(&prev);
   if (prev != p->device && cudaSetDevice(p->device) != cudaSuccess) return false;
-  k_upload<<<dim3((unsigned)n, (unsigned)n_frames), 256, 0, s>>>((const uint8_t *)a.devicePointer, (uint8_t *)dev,
-                                                                host_stride * es, dev_stride * es,
-                                                                (int64_t)p->ny * es, es, p->d_upload);
-  const bool ok = cudaGetLastError() == cudaSuccess;
+  const uint8_t *src = upload_source(p, host, es, n_frames, host_stride, dev, dev_stride);
+  bool ok = src != nullptr;
+  if (ok) {
+    k_upload<<<dim3((unsigned)p->upload_groups.size(), (unsigned)n_frames), 256, 0, s>>>(
+        src, (uint8_t *)dev, host_stride * es, dev_stride * es, (int64_t)p->ny * es, es, p->d_upload);
+    ok = cudaGetLastError() == cudaSuccess;
+  }
   if (prev != p->device) cudaSetDevice(prev);
   return ok;
 }

@@ -282,7 +282,9 @@ int mi_integrate_batch(mi_plan *plan, const void *frames, int dtype, int n_frame
  * frames are processed in chunks that fit the array; a plan needing more than the array
  * for one frame (n_r x 12 x 2 doubles > 1,048,576) gets MI_E_RANGE.  The first call on a
  * device looks up the array's address: make it before any stream capture.  Calls that
- * overlap on the GPU share the array and race.  A device reset while the library is loaded
+ * overlap on the GPU share the array and race.  Calls on a CSR plan use nothing of the plan and
+ * may overlap mi_integrate_batch on it; run and MMA plans stage frames in buffers of the plan,
+ * which calls of either kind share.  A device reset while the library is loaded
  * is not supported (the looked-up address is kept).  On a tensor-core (MMA) plan the chunk
  * is bounded by the array (11 frames per launch for 3960 x 360 bins), which costs speed. */
 int mi_integrate_batch_static(mi_plan *plan, const void *frames, int dtype, int n_frames,

@@ -341,7 +341,7 @@ int launch_lineout(Plan *p, const double *partial, int n_frames, double *lo_aw, 
 }
 
 int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t stride, float *cake,
-                double *lo_aw, double *lo_sm, double *partial, cudaStream_t s) {
+                double *lo_aw, double *lo_sm, double *partial, cudaStream_t s, bool fixed_scratch, double *res) {
   if (p->panels.size() > 1)
     return set_error(MI_E_ARG, "a panel plan takes its frames per panel: use mi_integrate_panels");
   CakeArgs a;
@@ -374,15 +374,18 @@ int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t st
   a.err = p->d_err;
   if (!a.want_cake && !a.want_lo) return MI_OK;
   int rc = MI_OK;
+  // a CSR plan's kernel writes nothing of the plan, which a call with scratch of its own relies on: the
+  // lane-per-bin kernels' bin results then need a place in that scratch
+  const bool no_res = fixed_scratch && p->encoding == MI_ENC_CSR && a.want_lo && !res;
   const bool mma = p->encoding == MI_ENC_MMA, u16 = dtype == MI_DT_U16 || dtype == MI_DT_U8;
   if ((mma ? u16 && n_frames >= kOnePmMinMma && n_frames <= kOnePmMma
            : n_frames >= kOnePmMin && (!u16 || n_frames <= kOnePmU16)) &&
       one_pm_fits(p, a.want_lo)) {
     // run and MMA plans: eight frames of a pixel side by side, a lane per bin (mi_one.cu)
     rc = launch_one_pm(p, &frames, &dtype, &stride, 0, n_frames, cake, partial, a.want_lo, s);
-  } else if (p->d_one_terms && n_frames <= (mma ? kOneFramesMma : kOneFrames) && (!mma || u16)) {
+  } else if (p->d_one_terms && n_frames <= (mma ? kOneFramesMma : kOneFrames) && (!mma || u16) && !no_res) {
     // few frames: a lane per bin, the same sums (mi_one.cu)
-    rc = launch_one(p, frames, dtype, n_frames, stride, cake, partial, a.want_lo, s);
+    rc = launch_one(p, frames, dtype, n_frames, stride, cake, partial, a.want_lo, res, s);
   } else if (p->encoding == MI_ENC_MMA) {
     // kernel (a) splits a chunk of frames into byte planes, then kernel (b) on the tensor cores
     if (!(dtype == MI_DT_U16 || dtype == MI_DT_U8))

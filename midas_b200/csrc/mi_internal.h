@@ -491,7 +491,8 @@ int build_host_csr(const mi_map_desc &m, int mode, int semantics, HostCSR *out);
 // `partial` is the lineout scratch, [n_frames][n_r][n_slots][2] doubles (the plan's d_partial,
 // or a caller-provided array of that size)
 int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t stride,
-                float *cake, double *lo_aw, double *lo_sm, double *partial, cudaStream_t s);
+                float *cake, double *lo_aw, double *lo_sm, double *partial, cudaStream_t s,
+                bool fixed_scratch = false, double *res = nullptr);
 // Up to kOneFrames frames of a run or CSR plan with a lane per bin (mi_one.cu); the same bits.
 // Run kernel / this, us: 16 frames 311 / 110 (1024^2, 495 x 45), 975 / 369 (2048^2, 990 x 72), 1101 /
 // 640 (2048^2, 1980 x 180 gradient), 1621 / 1114 (2880^2, 3960 x 360 gradient); 32 frames 318 / 218,
@@ -519,8 +520,9 @@ bool one_pm_fits(const Plan *p, bool want_lo);
 // frames [first, first + F) of every panel; cake and partial are those of the first
 int launch_one_pm(Plan *p, const void *const *frames, const int *dtypes, const int64_t *strides, int first, int F,
                   float *cake, double *partial, bool want_lo, cudaStream_t s);
+// res: the bin results of kOneChunk frames for the lineouts, null: the plan's own buffer
 int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
-               bool want_lo, cudaStream_t s);
+               bool want_lo, double *res, cudaStream_t s);
 int launch_runs(Plan *p, const void *frames, int dtype, int n_frames, int64_t stride, float *cake, double *partial,
                 bool want_lo, cudaStream_t s);
 // true when launch_runs stages this dtype through the pixel-major buffer

@@ -715,8 +715,9 @@ static OneArgs one_args(const Plan *p, int F, float *cake, double *res) {
 }
 
 static int launch_one_chunk(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
-                            bool want_lo, cudaStream_t s) {
-  double *res = !want_lo ? nullptr : (p->one_res_in_xc ? (double *)p->d_xc : p->d_one_res);
+                            bool want_lo, double *res, cudaStream_t s) {
+  if (!want_lo) res = nullptr;
+  else if (!res) res = p->one_res_in_xc ? (double *)p->d_xc : p->d_one_res;
   OneArgs a = one_args(p, F, cake, res);
   a.frames = frames;
   a.stride = stride;
@@ -739,13 +740,13 @@ static int launch_one_chunk(Plan *p, const void *frames, int dtype, int F, int64
 }
 
 int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, float *cake, double *partial,
-               bool want_lo, cudaStream_t s) {
+               bool want_lo, double *res, cudaStream_t s) {
   const size_t es = dtype_size(dtype);
   int rc = MI_OK;
   for (int f0 = 0; f0 < F && rc == MI_OK; f0 += kOneChunk)
     rc = launch_one_chunk(p, (const uint8_t *)frames + (size_t)f0 * stride * es, dtype, std::min(kOneChunk, F - f0),
                           stride, cake ? cake + (size_t)f0 * p->n_bins : nullptr,
-                          partial + (size_t)f0 * p->n_r * p->n_slots * 2, want_lo, s);
+                          partial + (size_t)f0 * p->n_r * p->n_slots * 2, want_lo, res, s);
   return rc;
 }
 

@@ -18,10 +18,13 @@
 // array: calls that overlap on the GPU (other streams, other threads) race on it.  Nothing
 // in it must start at zero: every launch writes every partial it later reads.  A call
 // copies nothing of the plan; it passes the array to the same launchers as
-// mi_integrate_batch.  On a tensor-core (MMA) plan the chunk is at most what the array
+// mi_integrate_batch.  A CSR plan's workspaces stay untouched, so such a call may overlap
+// mi_integrate_batch on the same plan; run and tensor-core plans stage frames in buffers of
+// their own and may not.  On a tensor-core (MMA) plan the chunk is at most what the array
 // holds (a 3960 x 360 bin plan with 12 partial slots per row: 11 frames per launch), and
 // that encoding's cost is per pass over the map, so such a plan runs slower per frame here
 // than through mi_integrate_batch.
+#include <algorithm>
 #include <mutex>
 
 #include "mi_internal.h"
@@ -80,11 +83,18 @@ extern "C" int mi_integrate_batch_static(mi_plan *p, const void *frames, int dty
     // the same launches as mi_integrate_batch, with the lineout partials in the fixed array
     const int chunk = (int)std::min<size_t>((size_t)kMaxFramesPerLaunch, kStaticScratchDoubles / per_frame);
     const size_t es = dtype_size(dtype);
+    // few frames of a CSR plan: the lane-per-bin kernels' bin results go behind the partial sums,
+    // where there is room (without it, the batched kernel), so that the call leaves the plan alone
+    const size_t n_res = (size_t)p->n_bins * kOneChunk;
+    double *res = nullptr;
+    if (p->encoding == MI_ENC_CSR && n_frames <= std::min(kOneFrames, chunk) &&
+        per_frame * n_frames + n_res <= kStaticScratchDoubles)
+      res = scratch + per_frame * n_frames;
     for (int f0 = 0; f0 < n_frames && rc == MI_OK; f0 += chunk) {
       const int nf = std::min(chunk, n_frames - f0);
       rc = launch_cake(p, (const uint8_t *)frames + (size_t)f0 * stride * es, dtype, nf, stride,
                        cake ? cake + (size_t)f0 * p->n_bins : nullptr, lo_aw ? lo_aw + (size_t)f0 * p->n_r : nullptr,
-                       lo_sm ? lo_sm + (size_t)f0 * p->n_r : nullptr, scratch, (cudaStream_t)stream);
+                       lo_sm ? lo_sm + (size_t)f0 * p->n_r : nullptr, scratch, (cudaStream_t)stream, true, res);
     }
   }
   if (prev != p->device) cudaSetDevice(prev);

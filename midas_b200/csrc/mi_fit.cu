@@ -445,9 +445,10 @@ extern "C" int mi_fit_batch(const double *x, const double *lineouts, int n_frame
   // then as many as keep every window of the call resident at once, up to 8 (14,080 windows:
   // 469 us with at most 4, 373 with 8, 372 with 16; 50,000: 1365, 1147, 1151)
   const uint32_t sb = fit_slot_bytes(2 * a.half + 1);
-  int dev = 0, sms = 0;
+  int dev = 0, sms = 0, dev_smem = 0;
   MI_CUDA(cudaGetDevice(&dev));
   MI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  MI_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const int64_t warps = (int64_t)sms * kFitWarps * 4;
   const int64_t fit = std::max<int64_t>(1, (48 * 1024 / kFitWarps) / sb);
   a.slots = (int)std::min<int64_t>(std::min<int64_t>(8, fit), (windows + warps - 1) / warps);
@@ -457,7 +458,7 @@ extern "C" int mi_fit_batch(const double *x, const double *lineouts, int n_frame
   const uint32_t smem = kFitWarps * (uint32_t)a.slots * sb;
   a.model = opts->model;
   auto kern = opts->model == MI_FIT_PV ? k_fit<MI_FIT_PV> : k_fit<MI_FIT_TCH>;
-  if (smem > 48 * 1024) MI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) MI_CUDA(allow_smem(kern, dev_smem));
   kern<<<(unsigned)blocks, 32 * kFitWarps, smem, (cudaStream_t)stream>>>(a);
   MI_CUDA(cudaGetLastError());
   return MI_OK;

@@ -1,9 +1,22 @@
 // mi_fitcore.cuh -- device helpers shared by the peak fitters (mi_fit.cu, mi_fitjob.cu).
 #pragma once
 
+#include <cuda_runtime.h>
 #include <math.h>
 
 namespace mi {
+
+// Let a kernel take all the shared memory the device has.  The limit belongs to the kernel, not to
+// a launch: set to each launch's own size, a thread with a smaller one between another's setting
+// and its launch would make that launch fail.
+template <typename K>
+inline cudaError_t allow_smem(K *kernel, int device_smem) {
+  cudaFuncAttributes f;
+  const cudaError_t e = cudaFuncGetAttributes(&f, kernel);
+  return e != cudaSuccess ? e
+                          : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 device_smem - (int)f.sharedSizeBytes);
+}
 
 __device__ inline double warp_sum(double v) {
 #pragma unroll

@@ -1185,13 +1185,13 @@ static int fit_plan_launch(const mi_fit_plan *fp, const FitPlanArgs &a, int64_t 
   k_fit_clear<<<(unsigned)((total + kClearSeries - 1) / kClearSeries), kClearSeries, 0, s>>>(a);
   MI_CUDA(cudaGetLastError());
   if (a.n_jobs > a.n_single) {
-    MI_CUDA(cudaFuncSetAttribute(k_fit_job, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MI_CUDA(allow_smem(k_fit_job, dev_smem));
     k_fit_job<<<(unsigned)((total + kJobWarps - 1) / kJobWarps), 32 * kJobWarps, smem, s>>>(a);
     MI_CUDA(cudaGetLastError());
   }
   if (units > 0) {
     const size_t es = (size_t)eta_warp_bytes(a.n_max, slots) * warps;
-    MI_CUDA(cudaFuncSetAttribute(k_fit_eta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)es));
+    MI_CUDA(allow_smem(k_fit_eta, dev_smem));
     k_fit_eta<<<(unsigned)blocks, 32 * warps, es, s>>>(a, slots);
     MI_CUDA(cudaGetLastError());
   }
@@ -1297,7 +1297,7 @@ extern "C" int mi_fit_autodetect(const double *x, const double *lineouts, int n_
   if (a.fit_warps < 1)
     return set_error(MI_E_RANGE, "mi_fit_autodetect: %d samples with +-%d-bin windows need %u B of shared memory",
                      n_x, roi_padding, total);
-  MI_CUDA(cudaFuncSetAttribute(k_fit_autodetect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)total));
+  MI_CUDA(allow_smem(k_fit_autodetect, dev_smem));
   k_fit_autodetect<<<(unsigned)n_frames, kAutoThreads, total, (cudaStream_t)stream>>>(a);
   MI_CUDA(cudaGetLastError());
   return MI_OK;

@@ -433,15 +433,22 @@ __global__ void k_map_trig(MapBins B, double *slo, double *clo, double *shi, dou
   chi[t] = cos(B.ehi[t] * kD2R);
 }
 
-// Records of every `step`-th pixel, summed: the size of the whole map within a few per cent.
+// Records of one pixel of every `step`, summed: the size of the whole map within a few per cent.  Two
+// samples, blockIdx.y: every step-th pixel, and one whose place in its group is mixed from the group's
+// number, so that a mask or module grid in step with the one is not with the other.
 __global__ void k_map_sample(MapGeom g, MapBins B, const uint8_t *mask, int step, unsigned long long *n_out) {
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * step;
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t h = k * 0x9E3779B1u;
+  h ^= h >> 15;
+  h *= 0x85EBCA77u;
+  h ^= h >> 13;
+  const int64_t t = (int64_t)k * step + (blockIdx.y ? h % (uint32_t)step : 0u);
   if (t >= (int64_t)g.ny * g.nz) return;
   const int i = (int)(t / g.nz), j = (int)(t % g.nz);
   if (mask && mask[(int64_t)j * g.ny + i]) return;
   unsigned long long n = 0;
   pixel_entries(g, B, i, j, false, [&](int32_t, const mi_map_record &) { ++n; }, [&](int32_t) {});
-  atomicAdd(n_out, n);
+  atomicAdd(n_out + blockIdx.y, n);
 }
 
 // Every pixel's records, in the order in which threads reach them: where they go in pixel order
@@ -678,29 +685,37 @@ static int build_device(const MapGeom &g, const MapBins &Bh, const uint8_t *mask
   MI_DCHK(dalloc((void **)&d_off, sizeof(int64_t) * (n_pix + 1)));
   MI_DCHK(dalloc((void **)&d_bmask, sizeof(int32_t) * n_bins));
   MI_DCHK(dalloc((void **)&d_bcnt, sizeof(int32_t) * n_bins));
-  MI_DCHK(dalloc((void **)&d_n, sizeof(unsigned long long)));
+  MI_DCHK(dalloc((void **)&d_n, 2 * sizeof(unsigned long long)));
   MI_DCHK(cudaMemsetAsync(d_bmask, 0, sizeof(int32_t) * n_bins, st));
   const int thr = 128;
   const unsigned grid = (unsigned)((n_pix + thr - 1) / thr);
-  // room for the entries: a sample's estimate and a tenth more; where that falls short, the
-  // count is known and the second run has room for all
+  // room for the entries: the smaller sample's estimate and a tenth more, at most what a map can hold;
+  // where that falls short or is not to be had, the records are counted and the second run has room for all
   constexpr int kStep = 67;
-  unsigned long long total_u = 0;
-  MI_DCHK(cudaMemsetAsync(d_n, 0, sizeof(unsigned long long), st));
-  k_map_sample<<<(unsigned)((n_pix / kStep + thr) / thr), thr, 0, st>>>(g, B, d_mask, kStep, d_n);
+  unsigned long long sample[2] = {0, 0}, total_u = 0;
+  MI_DCHK(cudaMemsetAsync(d_n, 0, sizeof(sample), st));
+  k_map_sample<<<dim3((unsigned)((n_pix / kStep + thr) / thr), 2), thr, 0, st>>>(g, B, d_mask, kStep, d_n);
   MI_DCHK(cudaGetLastError());
-  MI_DCHK(copy(&total_u, d_n, sizeof(total_u), cudaMemcpyDeviceToHost));
+  MI_DCHK(copy(sample, d_n, sizeof(sample), cudaMemcpyDeviceToHost));
   MapEntry *d_ent = nullptr;
-  unsigned long long cap = total_u * kStep + total_u * kStep / 10 + 65536;
+  const unsigned long long est = std::min(sample[0], sample[1]) * kStep;
+  unsigned long long cap = std::min<unsigned long long>(est + est / 10 + 65536, INT32_MAX);
   for (int run = 0; run < 2; ++run) {
-    MI_DCHK(dalloc((void **)&d_ent, sizeof(MapEntry) * cap));
+    const cudaError_t e = dalloc((void **)&d_ent, sizeof(MapEntry) * cap);
+    if (e != cudaSuccess && run == 0) {
+      cudaGetLastError();
+      cap = 0;   // counted only
+    } else {
+      MI_DCHK(e);
+    }
     MI_DCHK(cudaMemsetAsync(d_bcnt, 0, sizeof(int32_t) * n_bins, st));
     MI_DCHK(cudaMemsetAsync(d_n, 0, sizeof(unsigned long long), st));
     k_map_entries<<<grid, thr, 0, st>>>(g, B, d_mask, d_cnt, d_bmask, d_bcnt, d_ent, cap, d_n);
     MI_DCHK(cudaGetLastError());
     MI_DCHK(copy(&total_u, d_n, sizeof(total_u), cudaMemcpyDeviceToHost));
     if (total_u <= cap || total_u > INT32_MAX) break;
-    dfree(d_ent);
+    if (d_ent) dfree(d_ent);
+    d_ent = nullptr;
     cap = total_u;
   }
   if (total_u > INT32_MAX) {
@@ -724,7 +739,9 @@ static int build_device(const MapGeom &g, const MapBins &Bh, const uint8_t *mask
     k_map_place<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(d_ent, total, d_off, d_keys, d_recs);
     MI_DCHK(cudaGetLastError());
   }
-  dfree(d_ent);   // before the sort's buffers: the build needs no more memory than its records twice
+  // before the sort's buffers: the build's peak is here, 68 B a record and 4 B for each tenth of room over
+  // (entries 40, placed records and keys 28); the sort holds 64 B a record and its own scratch
+  if (d_ent) dfree(d_ent);
   MI_DCHK(dalloc((void **)&d_keys2, sizeof(int32_t) * total));
   MI_DCHK(dalloc((void **)&d_idx, sizeof(int32_t) * total));
   MI_DCHK(dalloc((void **)&d_idx2, sizeof(int32_t) * total));

@@ -439,7 +439,6 @@ struct Plan {
   int n_nan_bins = 0;
   float *d_dark = nullptr;       // ny*nz (zeros when no dark is set)
   int has_dark = 0;
-  int *d_has_dark = nullptr;     // the same on the device: a recorded graph follows a later dark
   int *d_err = nullptr;          // device error word (bounded waits)
   int *d_ctr = nullptr;          // work-item counter of the persistent run kernel
   int n_sms = 0;

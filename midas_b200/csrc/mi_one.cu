@@ -263,8 +263,7 @@ struct OneArgs {
   const double *scale;
   const void *frames;
   int64_t stride;
-  const float *dark;
-  const int *has_dark;      // 0: the dark is all zero and not read
+  const float *dark;        // null: none
   float *cake;              // [F][n_bins] or null
   double *res;              // [F / 8][n_bins][8] for the lineouts, or null
   int64_t n_bins;
@@ -294,7 +293,6 @@ __global__ void __launch_bounds__(128) k_one(OneArgs a) {
   const int64_t first = a.slice_ptr[s];
   int64_t at = first;
   const int f0 = (int)blockIdx.y * NF;
-  const float *dark = !INT && __ldg(a.has_dark) ? a.dark : nullptr;
   const T *img[NF];
   Acc acc[NF];
   double tot[NF];
@@ -316,7 +314,7 @@ __global__ void __launch_bounds__(128) k_one(OneArgs a) {
       const uint32_t p = t[u].x & ~kOneEnd;
 #pragma unroll
       for (int q = 0; q < NF; ++q) raw[u][q] = __ldg(img[q] + p);
-      d[u] = !INT && dark ? __ldg(dark + p) : 0.0f;
+      d[u] = !INT && a.dark ? __ldg(a.dark + p) : 0.0f;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -721,8 +719,10 @@ static int launch_one_chunk(Plan *p, const void *frames, int dtype, int F, int64
   OneArgs a = one_args(p, F, cake, res);
   a.frames = frames;
   a.stride = stride;
-  a.dark = p->d_dark;
-  a.has_dark = p->d_has_dark;
+  // without a dark its zeros are not read, except by a graph, which a later dark may follow
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (!p->has_dark) MI_CUDA(cudaStreamIsCapturing(s, &cap));
+  a.dark = cap == cudaStreamCaptureStatusNone ? nullptr : p->d_dark;
   int rc = MI_OK;
   if (p->encoding == MI_ENC_MMA) {
     rc = dtype == MI_DT_U8 ? launch_one_t<uint8_t, true>(p, a, s) : launch_one_t<uint16_t, true>(p, a, s);

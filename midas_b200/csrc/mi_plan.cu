@@ -574,7 +574,7 @@ static int free_plan_mem(Plan *p) {
                   p->d_ctr, p->d_span_lo, p->d_row_off, p->d_xchunks, p->d_xc,
                   p->d_xc_pix, p->d_nan_bins, p->d_upload,
                   p->d_one_cnt, p->d_one_ptr, p->d_one_terms, p->d_one_scale, p->d_one_tile,
-                  p->d_one_res, p->d_has_dark};
+                  p->d_one_res};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   return MI_OK;
@@ -1295,8 +1295,6 @@ static int build_plan(const mi_map_desc &m, const mi_plan_opts &o, Plan *p, Host
   MI_CUDA(cudaMalloc((void **)&p->d_dark, n_pix * sizeof(float)));
   MI_CUDA(cudaMemset(p->d_dark, 0, n_pix * sizeof(float)));
   acct += n_pix * sizeof(float);
-  MI_CUDA(cudaMalloc((void **)&p->d_has_dark, sizeof(int)));
-  MI_CUDA(cudaMemset(p->d_has_dark, 0, sizeof(int)));
   MI_CUDA(cudaMalloc((void **)&p->d_err, sizeof(int)));
   MI_CUDA(cudaMemset(p->d_err, 0, sizeof(int)));
   MI_CUDA(cudaMalloc((void **)&p->d_ctr, sizeof(int)));
@@ -1686,8 +1684,7 @@ int mi_plan_set_dark(mi_plan *p, const float *dark) {
   if (dark) MI_CUDA(copy_pieces(p->d_dark, dark, n * sizeof(float), cudaMemcpyHostToDevice));
   else MI_CUDA(cudaMemset(p->d_dark, 0, n * sizeof(float)));
   p->has_dark = dark ? 1 : 0;
-  MI_CUDA(cudaMemset(p->d_has_dark, p->has_dark, sizeof(int)));   // nonzero where set
-  MI_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // dark and flag have arrived, for any stream's kernels
+  MI_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // the dark has arrived, for any stream's kernels
   int rc = MI_OK;
   if (p->encoding == MI_ENC_MMA || p->encoding == MI_ENC_MMAD) {
     // the per-bin dark terms, computed once per dark on the legacy stream; waiting for that

@@ -340,6 +340,33 @@ int launch_lineout(Plan *p, const double *partial, int n_frames, double *lo_aw, 
   return MI_OK;
 }
 
+// the walk of the longest bin ends before the batched kernel (the lines' reasons: mi_internal.h)
+static bool lane_pays(const Plan *p, int n_frames) {
+  if (p->encoding == MI_ENC_MMA) {
+    const double ns = n_frames == 1 ? kMmaTermNs1
+                      : n_frames == 2 ? kMmaTermNs2
+                                      : kMmaTermNs + kMmaTermNsBlock * ((n_frames - 1) / kOneChunk);
+    return ns * (double)p->longest <= kMmaBaseNs + kMmaPixelNs * (double)p->staged_pixels;
+  }
+  if (p->encoding == MI_ENC_CSR) {
+    const int rest = n_frames % kOneChunk;
+    const double ns = kCsrTermNs * (n_frames / kOneChunk) + (rest == 0 ? 0.0 : rest <= 2 ? kCsrTermNs2 : kCsrTermNs);
+    return ns * (double)p->longest + kCsrBaseNs <= kCsrTileNs * p->depth;
+  }
+  return true;
+}
+
+CakeRoute cake_route(const Plan *p, int dtype, int n_frames, bool want_lo, bool lane_results) {
+  const bool mma = p->encoding == MI_ENC_MMA, u16 = dtype == MI_DT_U16 || dtype == MI_DT_U8;
+  if (!p->d_one_terms || (mma && !u16) || !lane_pays(p, n_frames)) return kRouteBatched;
+  // run and MMA plans: eight frames of a pixel side by side
+  if ((mma ? n_frames >= kOnePmMinMma && n_frames <= kOnePmMma
+           : n_frames >= kOnePmMin && (!u16 || n_frames <= kOnePmU16)) &&
+      one_pm_fits(p, want_lo))
+    return kRouteLaneEight;
+  return n_frames <= (mma ? kOneFramesMma : kOneFrames) && (!want_lo || lane_results) ? kRouteLane : kRouteBatched;
+}
+
 int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t stride, float *cake,
                 double *lo_aw, double *lo_sm, double *partial, cudaStream_t s, bool fixed_scratch, double *res) {
   if (p->panels.size() > 1)
@@ -377,13 +404,10 @@ int launch_cake(Plan *p, const void *frames, int dtype, int n_frames, int64_t st
   // a CSR plan's kernel writes nothing of the plan, which a call with scratch of its own relies on: the
   // lane-per-bin kernels' bin results then need a place in that scratch
   const bool no_res = fixed_scratch && p->encoding == MI_ENC_CSR && a.want_lo && !res;
-  const bool mma = p->encoding == MI_ENC_MMA, u16 = dtype == MI_DT_U16 || dtype == MI_DT_U8;
-  if ((mma ? u16 && n_frames >= kOnePmMinMma && n_frames <= kOnePmMma
-           : n_frames >= kOnePmMin && (!u16 || n_frames <= kOnePmU16)) &&
-      one_pm_fits(p, a.want_lo)) {
-    // run and MMA plans: eight frames of a pixel side by side, a lane per bin (mi_one.cu)
+  const CakeRoute route = cake_route(p, dtype, n_frames, a.want_lo, !no_res);
+  if (route == kRouteLaneEight) {
     rc = launch_one_pm(p, &frames, &dtype, &stride, 0, n_frames, cake, partial, a.want_lo, s);
-  } else if (p->d_one_terms && n_frames <= (mma ? kOneFramesMma : kOneFrames) && (!mma || u16) && !no_res) {
+  } else if (route == kRouteLane) {
     // few frames: a lane per bin, the same sums (mi_one.cu)
     rc = launch_one(p, frames, dtype, n_frames, stride, cake, partial, a.want_lo, res, s);
   } else if (p->encoding == MI_ENC_MMA) {

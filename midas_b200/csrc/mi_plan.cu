@@ -1275,6 +1275,7 @@ static int build_plan(const mi_map_desc &m, const mi_plan_opts &o, Plan *p, Host
     }
   }
   p->area_gs = csr.area_gs;
+  for (int64_t b = 0; b < p->n_bins; ++b) p->longest = std::max(p->longest, csr.row_ptr[b + 1] - csr.row_ptr[b]);
 
   size_t acct = 0;
   MI_CUDA(cudaSetDevice(p->device));
@@ -1299,6 +1300,8 @@ static int build_plan(const mi_map_desc &m, const mi_plan_opts &o, Plan *p, Host
   MI_CUDA(cudaMemset(p->d_err, 0, sizeof(int)));
   MI_CUDA(cudaMalloc((void **)&p->d_ctr, sizeof(int)));
   MI_CUDA(cudaDeviceGetAttribute(&p->n_sms, cudaDevAttrMultiProcessorCount, p->device));
+  p->depth = (p->n_tiles + std::max(p->n_sms, 1) - 1) / std::max(p->n_sms, 1);
+  for (const WorkItem &w : items) p->depth = std::max(p->depth, w.tile_end - w.tile_begin);
   if (n_xc > 0) {
     if ((rc = upload(&p->d_span_lo, span_lo.data(), span_lo.size(), &acct))) return rc;
     if ((rc = upload(&p->d_row_off, row_off.data(), row_off.size(), &acct))) return rc;
@@ -1926,6 +1929,11 @@ int mi_upload_frames(const mi_plan *p, const void *host, int dtype, int n_frames
 int mi_test_upload_by_kernel(const mi_plan *p, const void *host, int dtype, int n_frames, int64_t host_stride,
                              const void *device_frames, int64_t device_stride) {
   return upload_source(p, host, (int)dtype_size(dtype), n_frames, host_stride, device_frames, device_stride) != nullptr;
+}
+// and how mi_integrate_batch would cake a call's frames: 0 batched kernel, 1 lane per bin, 2 lane per bin
+// over eight frames of a pixel
+int mi_test_cake_route(const mi_plan *p, int dtype, int n_frames, int lineouts) {
+  return (int)cake_route(p, dtype, n_frames, lineouts && p->semantics != MI_SEM_OMP, true);
 }
 int mi_test_range_holds(uint64_t start, uint64_t bytes, uint64_t first, uint64_t last) {
   return range_holds(start, bytes, first, last);

@@ -376,13 +376,25 @@ class DeviceBackend:
         return g
 
     def footprint_estimate(self, cfg: StreamConfig) -> int:
-        """Upper estimate before building anything: map + staging + buffers."""
-        recs = cfg.pixmap.n_entries
-        B = cfg.max_batch or self.max_batch
+        """Upper estimate before building anything: map + staging + buffers.  Plans of 0.1 to 12 M
+        records, 8 to 102 a bin, hold 17 to 58 B a record in all modes and encodings besides the
+        partials, frames and staging below; with 2 a bin what a bin costs by itself shows."""
+        recs, bins, px = cfg.pixmap.n_entries, cfg.n_r * cfg.n_eta, cfg.n_pixels_y * cfg.n_pixels_z
+        B, enc = cfg.max_batch or self.max_batch, self.encoding_for(cfg)
         item = np.dtype(cfg.frame_dtype).itemsize
         ck = 8 if self.plain else (4 if cfg.want_cake else 0)
-        per_slot = B * (cfg.n_pixels_y * cfg.n_pixels_z * item + 16 * cfg.n_r + ck * cfg.n_r * cfg.n_eta)
-        plan = recs * 60 + 256 * cfg.n_r * 12 * 16 + cfg.n_pixels_y * cfg.n_pixels_z * 8
+        per_slot = B * (px * item + 16 * cfg.n_r + ck * bins)
+        if not self.plain:
+            per_slot += 8 * min(B, self.small_batch) * bins          # the one-frame kernel's FP64 cake
+        if cfg.peaks is not None:
+            per_slot += B * len(cfg.peaks) * (8 * L.FIT_NOUT + 4)
+        # lineout partials of 256 frames, 12 slots a row; the dark and one cast frame
+        plan = recs * 60 + bins * (96 if cfg.mode == "floor" else 160) + 256 * cfg.n_r * 12 * 16 + px * 8
+        if enc == "csr":
+            plan += 64 * bins + 64 * 1024                            # bin results of eight frames
+        elif enc in ("mma", "runs"):
+            # pixel-major staging of the referenced pixels, rows rounded out to 8
+            plan += 256 * min(px, 8 * recs * (1 if cfg.mode == "floor" else 4))
         return int(plan + self.max_inflight * per_slot)
 
     # -- staging at submission ------------------------------------------------------

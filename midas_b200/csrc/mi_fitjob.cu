@@ -340,21 +340,15 @@ __device__ void fit_one_job(const JobParams &c, const JobSmem &S, const FitJobDe
       for (int i = 0; i < n; ++i) mx = fmax(mx, S.y[i]);
       const double step = c.x_bin, gam0 = 3.0 * step;
       const double xfirst = xlo - xref, xlast = xhi - xref;
-      if (n_p == 1) {
-        const double c0 = pk_x[jd.p0] - xref;
-        S.p[0] = (float)c0;  S.lb[0] = (float)xfirst;  S.ub[0] = (float)xlast;
-        S.p[1] = (float)gam0;  S.lb[1] = (float)(step / 2);  S.ub[1] = (float)(step * n / 2);
-        S.p[2] = (float)(mx - bg0);  S.lb[2] = (float)((mx - bg0) / 100);  S.ub[2] = (float)(mx * 1.5);
-      } else {
-        double ig = mx - bg0;
-        if (ig < 1e-6) ig = 1e-6;
-        const double c1 = pk_x[jd.p0] - xref, c2 = pk_x[jd.p0 + 1] - xref, cm = 0.5 * (c1 + c2);
-        S.p[0] = (float)c1;  S.lb[0] = (float)xfirst;  S.ub[0] = (float)cm;
-        S.p[3] = (float)c2;  S.lb[3] = (float)cm;  S.ub[3] = (float)xlast;
-        for (int k = 0; k < 2; ++k) {
-          S.p[3 * k + 1] = (float)gam0;  S.lb[3 * k + 1] = (float)(step / 2);  S.ub[3 * k + 1] = (float)(step * n / 2);
-          S.p[3 * k + 2] = (float)(ig / 2);  S.lb[3 * k + 2] = (float)(ig / 100);  S.ub[3 * k + 2] = (float)(mx * 1.5);
-        }
+      // a doublet (pf_fit_doublet_pv); single peaks are k_fit_eta's
+      double ig = mx - bg0;
+      if (ig < 1e-6) ig = 1e-6;
+      const double c1 = pk_x[jd.p0] - xref, c2 = pk_x[jd.p0 + 1] - xref, cm = 0.5 * (c1 + c2);
+      S.p[0] = (float)c1;  S.lb[0] = (float)xfirst;  S.ub[0] = (float)cm;
+      S.p[3] = (float)c2;  S.lb[3] = (float)cm;  S.ub[3] = (float)xlast;
+      for (int k = 0; k < 2; ++k) {
+        S.p[3 * k + 1] = (float)gam0;  S.lb[3 * k + 1] = (float)(step / 2);  S.ub[3 * k + 1] = (float)(step * n / 2);
+        S.p[3 * k + 2] = (float)(ig / 2);  S.lb[3 * k + 2] = (float)(ig / 100);  S.ub[3 * k + 2] = (float)(mx * 1.5);
       }
       S.p[3 * n_p] = 0.5f;  S.lb[3 * n_p] = 0.0f;  S.ub[3 * n_p] = 1.0f;
       S.p[3 * n_p + 1] = (float)bg0;  S.lb[3 * n_p + 1] = 0.0f;
@@ -505,10 +499,11 @@ __global__ void __launch_bounds__(32 * kClearWarps) k_fit_clear(const FitPlanArg
 // iteration lane w solves unit w's damped normal equations, unrolled in registers, so the
 // serial FP64 chain runs for all the warp's units at once; then the whole warp evaluates one
 // unit after another, lane = sample, and forms J^T J and J^T r only of accepted steps.  The
-// model, the order of every sum and the iteration are fit_one_job's, bit for bit.
-// Bounded by FP64 issue and the solve's chain, not by memory.  fit_one_job (one column per warp,
-// the solve on lane 0 through shared memory) took 9.95 ms for 115,200 windows of 25 samples;
-// this takes 1.46 ms, same bits (1,800 windows of 19 samples: 2.56 -> 0.38 ms).
+// model, the order of every sum and the iteration are fit_one_job's.
+// Bounded by the solve's serial FP64 chain and the sums' issue, not by memory.  One
+// column per warp with the solve on lane 0 through shared memory, as the doublets are fit, took
+// 9.95 ms for 115,200 windows of 25 samples; this takes 1.46 ms, same bits (1,800 windows of 19
+// samples: 2.56 -> 0.38 ms).
 constexpr int kEtaNP = 5, kEtaTri = kEtaNP * (kEtaNP + 1) / 2, kEtaNrm = kEtaTri + kEtaNP;
 
 __host__ __device__ inline uint32_t eta_slot_bytes(int n_max) {

@@ -159,7 +159,9 @@ __host__ __device__ inline uint32_t fit_slot_bytes(int n_cap) {
 //   the TCH derivatives differently in their last bits, and the ill-conditioned (sig, gam)
 //   pair turns a last bit into another path of the iteration; evaluating both keeps the
 //   results of a fit what they always were.
-// What bounds it: the FP64 issue of the sums and the serial solve, not memory.  A solve by every
+// What bounds it: instruction issue and the fixed latencies of the serial solve at 21 % of the warps
+// (14,080 windows: issue slots 56 % busy, FP64 pipe 27, memory idle), and for a few windows the solve's
+// chain alone.  A solve by every
 // lane of a warp for its one window, all-reduced sums and two evaluations took 2.68 ms for
 // 14,080 PV windows of 31 samples; this takes 0.37 ms, and 80 us where it
 // took 160 for the 10 windows of one lineout (same bits).

@@ -500,8 +500,8 @@ __global__ void __launch_bounds__(32 * kClearWarps) k_fit_clear(const FitPlanArg
 // serial FP64 chain runs for all the warp's units at once; then the whole warp evaluates one
 // unit after another, lane = sample, and forms J^T J and J^T r only of accepted steps.  The
 // model, the order of every sum and the iteration are fit_one_job's.
-// Bounded by the solve's serial FP64 chain and the sums' issue, not by memory.  One
-// column per warp with the solve on lane 0 through shared memory, as the doublets are fit, took
+// Bounded by instruction issue, the chains of the solve and the sums and the trips through shared memory
+// at 23 % of the warps (115,200 windows: issue slots 55 % busy, FP64 pipe 19, DRAM idle).  One column per warp with the solve on lane 0 through shared memory, as the doublets are fit, took
 // 9.95 ms for 115,200 windows of 25 samples; this takes 1.46 ms, same bits (1,800 windows of 19
 // samples: 2.56 -> 0.38 ms).
 constexpr int kEtaNP = 5, kEtaTri = kEtaNP * (kEtaNP + 1) / 2, kEtaNrm = kEtaTri + kEtaNP;

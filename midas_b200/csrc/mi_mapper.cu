@@ -17,7 +17,7 @@
 // The geometry's FP64 functions are the cost.  Sines and cosines of the eta edges come from a
 // table, a corner's radius and angle are found once per pixel and not once per bin, a vertex's
 // once, and the candidate eta bins by bisection.  1475 x 1679 pixels, 790 x 72 bins: count and fill
-// pass 5.9 + 6.6 ms, now 4.7 + 0.1 (sample) + 0.1 ms.
+// pass 5.9 + 6.6 ms, now 4.7 + 0.1 (samples) + 0.1 ms.
 #include <cub/cub.cuh>
 #include <math.h>
 #include <omp.h>

@@ -273,9 +273,10 @@ struct OneArgs {
   const uint8_t *blobs;
 };
 
-// NF frames per pass over the map, U terms in flight per lane and as many fetched ahead.  Bounded
-// by the gathers (about one lane a clock and SM where a warp's pixels lie in different lines) and
-// at few bins by their latency.  One frame, cake only, where the run kernel took 298, 936, 1038 and
+// NF frames per pass over the map, U terms in flight per lane and as many fetched ahead.  Bounded by
+// the gathers' latency and issue together (one 2048^2 gradient frame: issue slots 65 % busy, L1 57, DRAM
+// 43, at 41 % of the warps) and at few bins by the latency alone (1024^2, 71,280 bins: 46, 35, 18 % at
+// 19 % of the warps).  One frame, cake only, where the run kernel took 298, 936, 1038 and
 // 1525 us: 33, 48, 67 and 112 us (1024^2, 495 x 45; 2048^2, 990 x 72; 1980 x 180 gradient; 2880^2,
 // 3960 x 360 gradient, 308 MB of terms).
 // INT (MMA encoding): integer weights, exact integer sums, the kernel's scaling.
@@ -369,10 +370,11 @@ __global__ void __launch_bounds__(128) k_one(OneArgs a) {
 //
 // Beyond a few frames the gathers bound k_one: a lane's pixels lie in different lines whatever a
 // line brings.  Here eight frames of a pixel lie side by side as fp32 minus the dark (one
-// sector), so a gather brings eight values and a term is read once for them.  Bounded by the
-// sectors from L2 (1475 x 1679 int32, 790 x 72 bins, 50 frames: 317 us for 29 M gathers, 2.9 TB/s) and by
-// the staging pass's bytes (150 us, 6 TB/s).  50 such frames with lineouts took 1078 us through the
-// 64-frame rows and the run kernel, 800 through k_one; 534 here.
+// sector), so a gather brings eight values and a term is read once for them.  Bounded by
+// the gathers' latency at few warps (1475 x 1679 int32, 790 x 72 bins, 50 frames: 317 us for 29 M
+// gathers, 2.9 TB/s from L2; 162 registers leave 17 % of the warps, with L1 58 % busy, L2 30, issue 22)
+// and by the staging pass's bytes (150 us, DRAM 65 % busy).  50 such frames with lineouts took 1078 us
+// through the 64-frame rows and the run kernel, 800 through k_one; 534 here.
 //
 // k_pm writes them: a thread per pixel of a span, eight coalesced loads, one 32-byte store.
 template <typename T>
@@ -399,7 +401,7 @@ __global__ void __launch_bounds__(256) k_pm(const T *__restrict__ frames, int64_
 }
 
 // the same for MMA plans: eight raw counts of 8/16-bit frames, 16 bytes a pixel (4 frames of 2048^2
-// gradient: 186 us through k_one, 116 with these)
+// gradient: 186 us through k_one, 116 with these; the sums L1 70 % busy, issue 53, at 40 % of the warps)
 template <typename T>
 __global__ void __launch_bounds__(256) k_pm16(const T *__restrict__ frames, int64_t stride, int F, int ny,
                                               const XcChunk *__restrict__ chunks, uint4 *__restrict__ pm, int64_t n_px) {

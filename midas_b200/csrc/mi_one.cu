@@ -756,7 +756,10 @@ int launch_one(Plan *p, const void *frames, int dtype, int F, int64_t stride, fl
 // mostly outside the panels' spans, else the detector's
 static int64_t pm_pixels(const Plan *p) { return p->panels.size() > 1 ? p->n_xc : (int64_t)p->ny * p->nz; }
 
-// eight-frame blocks that fit the pixel-major buffer together with their bin results
+// eight-frame blocks that fit the pixel-major buffer (256 B a referenced pixel) together with their bin
+// results.  None where the referenced band is under an eighth of the detector and twice the bins (32 B a
+// detector pixel for fp32), or the bins of a panel plan are over 3.5 a referenced pixel: over 16 wide
+// frames then go through the fp32 rows and the run kernel
 static int64_t pm_blocks(const Plan *p, bool want_lo) {
   const int64_t px = p->encoding == MI_ENC_MMA ? 2 : 4;   // bytes per pixel and frame
   const int64_t per = (pm_pixels(p) * px + (want_lo ? p->n_bins * 8 : 0)) * kPmFrames;

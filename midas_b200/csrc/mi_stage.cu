@@ -269,25 +269,31 @@ __global__ void __launch_bounds__(256) k_upload(const uint8_t *__restrict__ src,
   }
 }
 
-// The page-locked range that a host address lies in, from the driver (no link to libcuda)
-static bool locked_range(const void *ptr, uint64_t *start, uint64_t *bytes) {
-  using Fn = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+// A page-locked host address: its address on the device and the range it lies in, one query of the
+// driver (no link to libcuda).  False for any other memory.
+static bool locked_range(const void *ptr, uint64_t *dev, uint64_t *start, uint64_t *bytes) {
+  using Fn = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
   static const Fn query = [] {
     void *f = nullptr;
     cudaDriverEntryPointQueryResult q;
-    return cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+    return cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
                    q == cudaDriverEntryPointSuccess
                ? (Fn)f
                : nullptr;
   }();
-  CUdeviceptr at = 0;
+  CUmemorytype type{};
+  unsigned managed = 0;
+  CUdeviceptr at = 0, on_device = 0;
   size_t n = 0;
-  if (!query || query(&at, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)(uintptr_t)ptr) != CUDA_SUCCESS ||
-      query(&n, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)(uintptr_t)ptr) != CUDA_SUCCESS)
-    return false;
+  CUpointer_attribute want[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *got[] = {&type, &managed, &on_device, &at, &n};
+  if (!query || query(5, want, got, (CUdeviceptr)(uintptr_t)ptr) != CUDA_SUCCESS) return false;
+  *dev = (uint64_t)on_device;
   *start = (uint64_t)at;
   *bytes = (uint64_t)n;
-  return true;
+  return type == CU_MEMORYTYPE_HOST && !managed && on_device != 0;
 }
 
 bool range_holds(uint64_t start, uint64_t bytes, uint64_t first, uint64_t last) {
@@ -303,27 +309,20 @@ const uint8_t *upload_source(const Plan *p, const void *host, int es, int n_fram
   // every row is read as 16-byte pieces at one alignment on both sides
   if (((uintptr_t)host - (uintptr_t)dev) % 16 != 0) return nullptr;
   if (n_frames > 1 && ((host_stride - dev_stride) * es) % 16 != 0) return nullptr;
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
-  if ((uintptr_t)a.devicePointer % 16 != (uintptr_t)host % 16) return nullptr;
+  uint64_t src = 0, start = 0, bytes = 0;
+  if (!locked_range(host, &src, &start, &bytes) || src % 16 != (uintptr_t)host % 16) return nullptr;
   // one page-locked range holds the frames from the first byte to the last: buffers locked piece by
   // piece may have pageable memory between the pieces, and their device addresses do not tell
   const uint64_t first = (uint64_t)(uintptr_t)host;
   const uint64_t last = first + (uint64_t)(((int64_t)(n_frames - 1) * host_stride + (int64_t)p->ny * p->nz) * es) - 1;
-  uint64_t start = 0, bytes = 0;
-  if (!locked_range(host, &start, &bytes) || !range_holds(start, bytes, first, last)) return nullptr;
-  return (const uint8_t *)a.devicePointer;
+  return range_holds(start, bytes, first, last) ? (const uint8_t *)(uintptr_t)src : nullptr;
 }
 
 bool launch_upload(const Plan *p, const void *host, int es, int n_frames, int64_t host_stride, void *dev,
                    int64_t dev_stride, cudaStream_t s) {
   int prev = 0;
   cudaGetDevice(&prev);
-  if (prev != p->device && cudaSetDevice(p->device) != cudaSuccess) return false;
+  if (cudaSetDevice(p->device) != cudaSuccess) return false;   // also a thread's first call: the query needs a context
   const uint8_t *src = upload_source(p, host, es, n_frames, host_stride, dev, dev_stride);
   bool ok = src != nullptr;
   if (ok) {

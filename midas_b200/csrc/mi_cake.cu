@@ -349,8 +349,12 @@ static bool lane_pays(const Plan *p, int n_frames) {
     return ns * (double)p->longest <= kMmaBaseNs + kMmaPixelNs * (double)p->staged_pixels;
   }
   if (p->encoding == MI_ENC_CSR) {
-    const int rest = n_frames % kOneChunk;
-    const double ns = kCsrTermNs * (n_frames / kOneChunk) + (rest == 0 ? 0.0 : rest <= 2 ? kCsrTermNs2 : kCsrTermNs);
+    const double ns = n_frames == 1    ? kCsrTermNs1
+                      : n_frames == 2  ? kCsrTermNs2
+                      : n_frames <= 8  ? kCsrTermNs8
+                      : n_frames == 9  ? kCsrTermNs9
+                      : n_frames == 10 ? kCsrTermNs10
+                                       : kCsrTermNs16;
     return ns * (double)p->longest + kCsrBaseNs <= kCsrTileNs * p->depth;
   }
   return true;

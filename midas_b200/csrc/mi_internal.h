@@ -520,17 +520,18 @@ constexpr int kOnePmMinMma = 3, kOnePmMma = 24;
 // kernels spread a tile's pixels over a block, so the frame counts above hold where the longest bin's
 // walk ends before they do.  In ns, fitted to 157 plans (128^2 to 2048^2 pixels, 45 to 356,400 bins of
 // 32 to 1777 terms, 0.07 to 18 M terms) at 1 to 24 frames; no plan is over 3 % (MMA) and 6 % (CSR) slower
-// by it than by the batched kernel, and by 1 % and 2 % on average than by the better of the two:
+// by it than by the batched kernel, and by 1 % on average than by the better of the two:
 // MMA: the walk a term, by frames, against 12 us and the pixels the tiles stage.  Batched / lane per
 //   bin, us, 4 frames: 1777 terms (256^2, 124 x 1) 47 / 245; 714 (1024^2, 124 x 24) 137 / 121; 321 (512^2,
 //   248 x 12) 74 / 65; 178 (1024^2, 495 x 45) 148 / 49.
-// CSR: the walk a term and chunk of eight frames, by its frames, against the tiles in sequence.  16
-//   frames: 321 terms, 8 tiles (512^2, 248 x 12) 93 / 204; 636, 20 (1024^2, 495 x 12) 286 / 384; 106, 61
-//   (2048^2, 1980 x 180 gradient) 1042 / 456; 4 frames 78 / 105, 241 / 195, 747 / 141.
+// CSR: the walk a term, by frames (eight at a time), against the tiles in sequence.  16 frames: 321
+//   terms, 8 tiles (512^2, 248 x 12) 93 / 204; 636, 20 (1024^2, 495 x 12) 286 / 384; 106, 61 (2048^2,
+//   1980 x 180 gradient) 1042 / 456; 4 frames 78 / 105, 241 / 195, 747 / 141.
 // The run kernel's walk is long itself: it was the faster one by over 7 us in no plan.
 constexpr double kMmaTermNs1 = 38, kMmaTermNs2 = 100, kMmaTermNs = 125, kMmaTermNsBlock = 25;
 constexpr double kMmaBaseNs = 12000, kMmaPixelNs = 0.088;
-constexpr double kCsrTermNs2 = 100, kCsrTermNs = 310, kCsrBaseNs = 20000, kCsrTileNs = 7500;
+constexpr double kCsrTermNs1 = 20, kCsrTermNs2 = 50, kCsrTermNs8 = 170, kCsrTermNs9 = 300, kCsrTermNs10 = 340,
+                 kCsrTermNs16 = 470, kCsrBaseNs = 18000, kCsrTileNs = 6000;
 enum CakeRoute { kRouteBatched = 0, kRouteLane = 1, kRouteLaneEight = 2 };
 // which kernels cake n_frames of a plan of one detector (mi_cake.cu); lane_results: the lane-per-bin
 // kernels have a place for the bin results of the lineouts

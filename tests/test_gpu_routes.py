@@ -37,7 +37,7 @@ def _route(plan, dt, n, lineouts=True):
 
 
 # by the lines of the rule (mi_internal.h): a walk a term and frame count against 12 us and 0.088 ns a
-# staged pixel (MMA; the maps stage 100 to 36,000 pixels, at most 3.2 us) or 7.5 us a tile in sequence (CSR)
+# staged pixel (MMA; the maps stage 100 to 36,000 pixels, at most 3.2 us) or 6 us a tile in sequence (CSR)
 @pytest.mark.parametrize("n_r,n_eta,terms,lane", [
     (2, 1, 1700, ()),                            # 64.6 us at one frame
     (2, 3, 450, ()),                             # 17.1
@@ -53,8 +53,8 @@ def test_mma_plans(cuda, n_r, n_eta, terms, lane):
 
 
 # one band of rows, so all tiles follow one another: 100 and 300 terms a bin over few tiles, the batched kernel
-# for most counts; 14 or 15 terms over tiles of 64 pixels (30 or more), a lane per bin for all
-@pytest.mark.parametrize("n_eta,lo,hi,pixels", [(1, 95, 100, 0), (1, 295, 300, 0), (8, 14, 16, 64)])
+# for most counts; 30 to 39 terms over tiles of 64 pixels, about 20 in an item of two columns, a lane per bin for all
+@pytest.mark.parametrize("n_eta,lo,hi,pixels", [(1, 95, 100, 0), (1, 295, 300, 0), (24, 30, 40, 64)])
 def test_csr_plans(cuda, n_eta, lo, hi, pixels):
     plan = _plan(cuda, "csr", 16, n_eta, lo, hi, tile_pixels=pixels, tile_rows=16)
     assert plan.info["n_items"] == 1 or pixels
@@ -62,8 +62,8 @@ def test_csr_plans(cuda, n_eta, lo, hi, pixels):
     seen = set()
     for dt in (torch.uint16, torch.float32):
         for n in (1, 2, 3, 8, 9, 16, 17, 128):
-            walk = sum({1: 0.1, 2: 0.1}.get(min(8, n - f), 0.31) for f in range(0, n, 8)) * (hi - 1)
-            want = LANE if n <= 16 and (pixels or walk + 20 <= 7.5 * tiles) else BATCHED
+            walk = {1: 0.02, 2: 0.05, 3: 0.17, 8: 0.17, 9: 0.3, 16: 0.47}.get(n, 0) * (hi - 1)
+            want = LANE if n <= 16 and (pixels or walk + 18 <= 6 * tiles) else BATCHED
             seen.add((n, want))
             assert _route(plan, dt, n) == want, (n, tiles)
     assert ((16, BATCHED) in seen) == (not pixels) and (17, BATCHED) in seen
@@ -81,10 +81,10 @@ def test_run_plans(cuda, n_r, n_eta):
 
 @pytest.mark.parametrize("mode,sem,norm,var", [("floor", "py", True, False), ("gradient", "py", False, True),
                                                ("bilinear", "gpustream", False, False), ("gradient", "ic", True, False)])
-@pytest.mark.parametrize("n_r,n_eta", [(16, 8), (37, 5)])
+@pytest.mark.parametrize("n_r,n_eta", [(16, 24), (37, 27)])
 def test_csr_lane_equals_batched(cuda, mode, sem, norm, var, n_r, n_eta):
     """small tiles, many in sequence: a lane per bin for up to 16 frames"""
-    plan = _plan(cuda, "csr", n_r, n_eta, 8, 16, tile_pixels=64, mode=mode, semantics=sem, normalize=norm, variance=var)
+    plan = _plan(cuda, "csr", n_r, n_eta, 30, 40, tile_pixels=64 if mode == "floor" else 256, mode=mode, semantics=sem, normalize=norm, variance=var)
     rng = np.random.default_rng(n_r)
     raw = rng.integers(0, 250, (40, 190, 201))
     for dark in (None, rng.normal(100, 5, (190, 201))):
